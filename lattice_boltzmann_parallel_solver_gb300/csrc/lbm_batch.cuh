@@ -138,12 +138,16 @@ __global__ void __launch_bounds__(THREADS, batch_min_blocks<STORE, NPT, THREADS,
   const int per = total_tiles / (int)gridDim.x, extra = total_tiles % (int)gridDim.x;
   const int b = (int)blockIdx.x;
   const int t0 = b * per + min(b, extra), t1 = t0 + per + (b < extra ? 1 : 0);
-  if (t0 >= t1) return;
+  if (t0 >= t1) {
+    pdl_wait();
+    return;
+  }
   const int g = *gbase + k;
   int lo = owner_of(tile_start, n_inst, t0);
   int first = __ldg(tile_start + lo);
   int next = lo + 1 < n_inst ? __ldg(tile_start + lo + 1) : total_tiles;
   stage_entry<THREADS, HAS_BC>(tab, lo, ebuf);
+  pdl_wait();  // the table and the global step are not written during a run
   for (int tile = t0; tile < t1; ++tile) {
     if (tile >= next) {
       do {
@@ -190,6 +194,7 @@ __global__ void __launch_bounds__(THREADS, batch_min_blocks<STORE, NPT, THREADS,
   const int lo = owner_of_staged<THREADS>(tile_start, n_inst, tile);
   stage_entry<THREADS, HAS_BC>(tab, lo, ebuf);
   const int g = *gbase + k;
+  pdl_wait();  // the table and the global step are not written during a run
   if (g < e.s0 || g >= e.s_end) return;
   batch_tile<STORE, NPT, THREADS, HAS_BC, SHIFT>(e, tile - __ldg(tile_start + lo), g);
 }
@@ -225,6 +230,7 @@ __global__ void __launch_bounds__(kFixupChunk, STORE == LBM_STORE_FX64 ? 1 : 8)
   const int g = *gbase + k;
   const int j = owner_of_staged<kFixupChunk>(bc_start, n_inst, (int)blockIdx.x);
   stage_entry<kFixupChunk, true>(tab, j, ebuf);
+  pdl_wait();
   if (g < e.s0 || g >= e.s_end) return;
   const int t = ((int)blockIdx.x - __ldg(bc_start + j)) * kFixupChunk + (int)threadIdx.x;
   const int nx = e.P.g.nx;
@@ -292,16 +298,19 @@ inline int launch_batch(const void* table, int n, int tiles, int bc_chunks, int*
   blocks = std::min(blocks, std::max(1, tiles));
   for (int k = 0; k < nsteps; ++k) {
     if (plain && tiles > 0) {
-      batch_grid_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT><<<tiles, THREADS, 0, s>>>(tab, start, n, gbase, k);
+      launch_step(batch_grid_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT>, dim3((unsigned)tiles), THREADS, k > 0, s, tab,
+                  start, n, (const int*)gbase, k);
       count_launch();
       if (int e = check_launch("batch_grid_kernel")) return e;
     } else {
-      batch_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT><<<blocks, THREADS, 0, s>>>(tab, start, n, tiles, gbase, k);
+      launch_step(batch_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT>, dim3((unsigned)blocks), THREADS, k > 0, s, tab, start,
+                  n, tiles, (const int*)gbase, k);
       count_launch();
       if (int e = check_launch("batch_kernel")) return e;
     }
     if (!HAS_BC && bc_chunks > 0) {
-      batch_fixup_kernel<STORE, SHIFT><<<bc_chunks, kFixupChunk, 0, s>>>(tab, bc_start, n, gbase, k);
+      launch_step(batch_fixup_kernel<STORE, SHIFT>, dim3((unsigned)bc_chunks), kFixupChunk, true, s, tab, bc_start, n,
+                  (const int*)gbase, k);
       count_launch();
       if (int e = check_launch("batch_fixup_kernel")) return e;
     }

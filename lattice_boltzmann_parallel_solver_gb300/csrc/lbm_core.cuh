@@ -33,13 +33,15 @@ static_assert(opp(5) == 7 && opp(6) == 8 && opp(7) == 5 && opp(8) == 6, "opp");
 __host__ __device__ constexpr int outlet_slot(int i) { return i == 3 ? 0 : (i == 6 ? 1 : (i == 7 ? 2 : -1)); }
 
 // ---------------------------------------------------------------------------
-// storage of the resident populations
+// storage of the resident populations.  Populations are read by plain loads,
+// not through the read-only path: a step's kernel may start while the one
+// before it still writes them (pdl_wait).
 // ---------------------------------------------------------------------------
 template <int S> struct Store;
 template <> struct Store<LBM_STORE_F64> {
   using T = double;
   using R = double;
-  __device__ static R ld(const T* p, int) { return __ldg(p); }
+  __device__ static R ld(const T* p, int) { return *p; }
   __device__ static void st(T* p, R v, int) { *p = v; }
   __device__ static R to_r(T t, int) { return t; }
   __device__ static T from_r(R v, int) { return v; }
@@ -51,7 +53,7 @@ template <> struct Store<LBM_STORE_F64> {
 template <> struct Store<LBM_STORE_F32> {
   using T = float;
   using R = float;
-  __device__ static R ld(const T* p, int) { return __ldg(p); }
+  __device__ static R ld(const T* p, int) { return *p; }
   __device__ static void st(T* p, R v, int) { *p = v; }
   __device__ static R to_r(T t, int) { return t; }
   __device__ static T from_r(R v, int) { return v; }
@@ -67,7 +69,7 @@ template <> struct Store<LBM_STORE_FX64> {
   using T = long long;
   using R = double;
   using A = long long;
-  __device__ static R ld(const T* p, int i) { return fx::from_fx(__ldg(p), wd(i)); }
+  __device__ static R ld(const T* p, int i) { return fx::from_fx(*p, wd(i)); }
   __device__ static void st(T* p, R v, int i) { *p = fx::to_fx(v, wd(i)); }
   __device__ static R to_r(T t, int i) { return fx::from_fx(t, wd(i)); }
   __device__ static T from_r(R v, int i) { return fx::to_fx(v, wd(i)); }
@@ -83,7 +85,7 @@ template <> struct Store<LBM_STORE_F16S> {
   using T = __half;
   using R = float;
   static constexpr float kScale = 1024.0f, kInv = 1.0f / 1024.0f;
-  __device__ static R ld(const T* p, int i) { return fmaf(__half2float(__ldg(p)), kInv, wf(i)); }
+  __device__ static R ld(const T* p, int i) { return fmaf(__half2float(*p), kInv, wf(i)); }
   __device__ static void st(T* p, R v, int i) { *p = __float2half_rn((v - wf(i)) * kScale); }
   __device__ static R to_r(T t, int i) { return fmaf(__half2float(t), kInv, wf(i)); }
   __device__ static T from_r(R v, int i) { return __float2half_rn((v - wf(i)) * kScale); }
@@ -94,7 +96,7 @@ template <> struct Store<LBM_STORE_F16S> {
   // the vectorised kernel works on the stored, scaled deviation D = 1024 (f_i - w_i)
   static constexpr float kDev = kScale;
   __device__ static R dev(T t) { return __half2float(t); }
-  __device__ static R ld_dev(const T* p) { return __half2float(__ldg(p)); }
+  __device__ static R ld_dev(const T* p) { return __half2float(*p); }
   __device__ static T dev_rn(R d) { return __float2half_rn(d); }
   // stochastic rounding: the top 13 bits of r, added below the 10 mantissa bits
   // binary16 keeps, then truncation
@@ -105,7 +107,7 @@ template <> struct Store<LBM_STORE_F16S> {
 template <> struct Store<LBM_STORE_BF16S> {
   using T = __nv_bfloat16;
   using R = float;
-  __device__ static R ld(const T* p, int i) { return wf(i) + __bfloat162float(__ldg(p)); }
+  __device__ static R ld(const T* p, int i) { return wf(i) + __bfloat162float(*p); }
   __device__ static void st(T* p, R v, int i) { *p = __float2bfloat16_rn(v - wf(i)); }
   __device__ static R to_r(T t, int i) { return wf(i) + __bfloat162float(t); }
   __device__ static T from_r(R v, int i) { return __float2bfloat16_rn(v - wf(i)); }
@@ -115,7 +117,7 @@ template <> struct Store<LBM_STORE_BF16S> {
   static constexpr bool kShifted = true;
   static constexpr float kDev = 1.0f;  // working deviation: f_i - w_i
   __device__ static R dev(T t) { return __bfloat162float(t); }
-  __device__ static R ld_dev(const T* p) { return __bfloat162float(__ldg(p)); }
+  __device__ static R ld_dev(const T* p) { return __bfloat162float(*p); }
   __device__ static T dev_rn(R d) { return __float2bfloat16_rn(d); }
   // stochastic rounding: the top 16 bits of r, added below the 16 bits bfloat16
   // keeps, then truncation
@@ -152,14 +154,14 @@ __device__ __forceinline__ void ld_vec(const T* p, T out[N]) {
   if constexpr (B % 16 == 0) {
 #pragma unroll
     for (int j = 0; j < B / 16; ++j) {
-      const uint4 t = __ldg(reinterpret_cast<const uint4*>(p) + j);
+      const uint4 t = reinterpret_cast<const uint4*>(p)[j];
       memcpy(&out[j * (16 / sizeof(T))], &t, 16);
     }
   } else if constexpr (B == 8) {
-    const uint2 t = __ldg(reinterpret_cast<const uint2*>(p));
+    const uint2 t = *reinterpret_cast<const uint2*>(p);
     memcpy(out, &t, 8);
   } else if constexpr (B == 4) {
-    const unsigned t = __ldg(reinterpret_cast<const unsigned*>(p));
+    const unsigned t = *reinterpret_cast<const unsigned*>(p);
     memcpy(out, &t, 4);
   } else {
 #pragma unroll

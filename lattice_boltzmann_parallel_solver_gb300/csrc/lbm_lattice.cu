@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(THREADS, (STORE == LBM_STORE_F16S || STORE == 
                                                ? 1024 / THREADS
                                                : 1)
     fused_v2_kernel(const __grid_constant__ KParams P) {
+  pdl_wait();
   fused_v2_body<STORE, NPT, HAS_BC, HAS_PRESSURE, false, SHIFT>(P, P.pop_in, P.pop_out, P.aux_in, P.aux_out,
                                                                 (blockIdx.x * THREADS + threadIdx.x) * NPT,
                                                                 blockIdx.y, launch_seed(P));
@@ -206,6 +207,7 @@ __global__ void __launch_bounds__(THREADS, (STORE == LBM_STORE_F16S || STORE == 
 // one node per thread: registers capped so that 1024 threads fit on an SM
 template <int NPT, int THREADS, bool HAS_BC, bool HAS_PRESSURE>
 __global__ void __launch_bounds__(THREADS, NPT == 1 ? 1024 / THREADS : 1) fused_fx_kernel(const __grid_constant__ KParams P) {
+  pdl_wait();
   fused_fx_body<NPT, HAS_BC, HAS_PRESSURE>(P, P.pop_in, P.pop_out, P.aux_in, P.aux_out,
                                            (blockIdx.x * THREADS + threadIdx.x) * NPT, blockIdx.y);
 }
@@ -216,6 +218,7 @@ __global__ void __launch_bounds__(THREADS, NPT == 1 ? 1024 / THREADS : 1) fused_
 // the random bits are those of the in-step path) and overwrites its outputs.
 template <int STORE, int THREADS, bool HAS_PRESSURE, bool SHIFT>
 __global__ void __launch_bounds__(THREADS) fixup_v2_kernel(const __grid_constant__ KParams P) {
+  pdl_wait();
   const int t = blockIdx.x * THREADS + threadIdx.x;
   if (t >= P.g.n_bcnodes) return;
   const int node = __ldg(P.g.bcnodes + t);
@@ -278,13 +281,13 @@ constexpr int kV2Threads = 128;
   do {                                                                                 \
     const bool bc = P.g.bcmask != nullptr, pr = P.g.pressure != 0;                     \
     if (bc && pr)                                                                      \
-      KERNEL<__VA_ARGS__, true, true><<<grid, kV2Threads, 0, s>>>(P);                  \
+      launch_step(KERNEL<__VA_ARGS__, true, true>, grid, kV2Threads, overlap, s, P);   \
     else if (bc)                                                                       \
-      KERNEL<__VA_ARGS__, true, false><<<grid, kV2Threads, 0, s>>>(P);                 \
+      launch_step(KERNEL<__VA_ARGS__, true, false>, grid, kV2Threads, overlap, s, P);  \
     else if (pr)                                                                       \
-      KERNEL<__VA_ARGS__, false, true><<<grid, kV2Threads, 0, s>>>(P);                 \
+      launch_step(KERNEL<__VA_ARGS__, false, true>, grid, kV2Threads, overlap, s, P);  \
     else                                                                               \
-      KERNEL<__VA_ARGS__, false, false><<<grid, kV2Threads, 0, s>>>(P);                \
+      launch_step(KERNEL<__VA_ARGS__, false, false>, grid, kV2Threads, overlap, s, P); \
   } while (0)
 
 template <int NPT>
@@ -294,7 +297,7 @@ static dim3 v2_grid(const KParams& P) {
 }
 
 template <int STORE, int NPT, bool SHIFT = false>
-static int launch_v2(const KParams& P, cudaStream_t s) {
+static int launch_v2(const KParams& P, bool overlap, cudaStream_t s) {
   const dim3 grid = v2_grid<NPT>(P);
   LBM_LAUNCH_SPECIALISED(fused_v2_kernel, STORE, NPT, kV2Threads, SHIFT);
   count_launch();
@@ -302,7 +305,7 @@ static int launch_v2(const KParams& P, cudaStream_t s) {
 }
 
 template <int NPT>
-static int launch_fx(const KParams& P, cudaStream_t s) {
+static int launch_fx(const KParams& P, bool overlap, cudaStream_t s) {
   const dim3 grid = v2_grid<NPT>(P);
   LBM_LAUNCH_SPECIALISED(fused_fx_kernel, NPT, kV2Threads);
   count_launch();
@@ -334,17 +337,18 @@ static int v2_npt(int storage, int flags, const KParams& P) {
 constexpr int kFixupThreads = 128;
 
 template <int STORE, bool SHIFT = false>
+// (always right after the step kernel of the same launch_fused)
 static int launch_fixup(const KParams& P, cudaStream_t s) {
   const dim3 grid((unsigned)((P.g.n_bcnodes + kFixupThreads - 1) / kFixupThreads));
   if (P.g.pressure)
-    fixup_v2_kernel<STORE, kFixupThreads, true, SHIFT><<<grid, kFixupThreads, 0, s>>>(P);
+    launch_step(fixup_v2_kernel<STORE, kFixupThreads, true, SHIFT>, grid, kFixupThreads, true, s, P);
   else
-    fixup_v2_kernel<STORE, kFixupThreads, false, SHIFT><<<grid, kFixupThreads, 0, s>>>(P);
+    launch_step(fixup_v2_kernel<STORE, kFixupThreads, false, SHIFT>, grid, kFixupThreads, true, s, P);
   count_launch();
   return check_launch("fixup_v2_kernel");
 }
 
-static int launch_fused_step(int storage, int npt, int flags, const KParams& P, cudaStream_t s);
+static int launch_fused_step(int storage, int npt, int flags, const KParams& P, bool overlap, cudaStream_t s);
 
 // One step.  On large lattices whose geometry lists its boundary nodes (at most
 // an eighth of the lattice), the vectorised kernel runs without boundary work:
@@ -360,7 +364,7 @@ static int64_t split_nodes(int storage) {
                                                                                               : (int64_t)1 << 25;
 }
 
-static int launch_fused(int storage, int flags, const KParams& P, cudaStream_t s) {
+static int launch_fused(int storage, int flags, const KParams& P, bool overlap, cudaStream_t s) {
   const int npt = v2_npt(storage, flags, P);
   const int64_t nodes = (int64_t)P.g.nx * P.g.ny;
   // a probe keeps the sources inside the step, so its node is recorded once
@@ -368,10 +372,10 @@ static int launch_fused(int storage, int flags, const KParams& P, cudaStream_t s
                      P.probe_buf == nullptr &&
                      (nodes >= split_nodes(storage) || (flags & LBM_FLAG_BC_SPLIT)) &&
                      (int64_t)P.g.n_bcnodes * 8 <= nodes;
-  if (!split) return launch_fused_step(storage, npt, flags, P, s);
+  if (!split) return launch_fused_step(storage, npt, flags, P, overlap, s);
   KParams Q = P;
   Q.g.bcmask = nullptr;
-  if (int e = launch_fused_step(storage, npt, flags, Q, s)) return e;
+  if (int e = launch_fused_step(storage, npt, flags, Q, overlap, s)) return e;
   switch (storage) {
     case LBM_STORE_F64: return launch_fixup<LBM_STORE_F64>(P, s);
     case LBM_STORE_F32: return launch_fixup<LBM_STORE_F32>(P, s);
@@ -384,23 +388,23 @@ static int launch_fused(int storage, int flags, const KParams& P, cudaStream_t s
   }
 }
 
-static int launch_fused_step(int storage, int npt, int flags, const KParams& P, cudaStream_t s) {
+static int launch_fused_step(int storage, int npt, int flags, const KParams& P, bool overlap, cudaStream_t s) {
   switch (storage * 16 + npt) {
-    case LBM_STORE_F64 * 16 + 2: return launch_v2<LBM_STORE_F64, 2>(P, s);
-    case LBM_STORE_F64 * 16 + 4: return launch_v2<LBM_STORE_F64, 4>(P, s);
-    case LBM_STORE_FX64 * 16 + 1: return launch_fx<1>(P, s);
-    case LBM_STORE_FX64 * 16 + 2: return launch_fx<2>(P, s);
-    case LBM_STORE_FX64 * 16 + 4: return launch_fx<4>(P, s);
-    case LBM_STORE_F32 * 16 + 2: return launch_v2<LBM_STORE_F32, 2>(P, s);
-    case LBM_STORE_F32 * 16 + 4: return launch_v2<LBM_STORE_F32, 4>(P, s);
-    case LBM_STORE_F16S * 16 + 2: return launch_v2<LBM_STORE_F16S, 2>(P, s);
-    case LBM_STORE_F16S * 16 + 4: return launch_v2<LBM_STORE_F16S, 4>(P, s);
-    case LBM_STORE_F16S * 16 + 8: return launch_v2<LBM_STORE_F16S, 8>(P, s);
-    case LBM_STORE_BF16S * 16 + 2: return launch_v2<LBM_STORE_BF16S, 2>(P, s);
-    case LBM_STORE_BF16S * 16 + 4: return launch_v2<LBM_STORE_BF16S, 4>(P, s);
-    case LBM_STORE_BF16S * 16 + 8: return launch_v2<LBM_STORE_BF16S, 8>(P, s);
-    case LBM_STORE_F16R * 16 + 4: return launch_v2<LBM_STORE_F16S, 4, true>(P, s);
-    case LBM_STORE_BF16R * 16 + 4: return launch_v2<LBM_STORE_BF16S, 4, true>(P, s);
+    case LBM_STORE_F64 * 16 + 2: return launch_v2<LBM_STORE_F64, 2>(P, overlap, s);
+    case LBM_STORE_F64 * 16 + 4: return launch_v2<LBM_STORE_F64, 4>(P, overlap, s);
+    case LBM_STORE_FX64 * 16 + 1: return launch_fx<1>(P, overlap, s);
+    case LBM_STORE_FX64 * 16 + 2: return launch_fx<2>(P, overlap, s);
+    case LBM_STORE_FX64 * 16 + 4: return launch_fx<4>(P, overlap, s);
+    case LBM_STORE_F32 * 16 + 2: return launch_v2<LBM_STORE_F32, 2>(P, overlap, s);
+    case LBM_STORE_F32 * 16 + 4: return launch_v2<LBM_STORE_F32, 4>(P, overlap, s);
+    case LBM_STORE_F16S * 16 + 2: return launch_v2<LBM_STORE_F16S, 2>(P, overlap, s);
+    case LBM_STORE_F16S * 16 + 4: return launch_v2<LBM_STORE_F16S, 4>(P, overlap, s);
+    case LBM_STORE_F16S * 16 + 8: return launch_v2<LBM_STORE_F16S, 8>(P, overlap, s);
+    case LBM_STORE_BF16S * 16 + 2: return launch_v2<LBM_STORE_BF16S, 2>(P, overlap, s);
+    case LBM_STORE_BF16S * 16 + 4: return launch_v2<LBM_STORE_BF16S, 4>(P, overlap, s);
+    case LBM_STORE_BF16S * 16 + 8: return launch_v2<LBM_STORE_BF16S, 8>(P, overlap, s);
+    case LBM_STORE_F16R * 16 + 4: return launch_v2<LBM_STORE_F16S, 4, true>(P, overlap, s);
+    case LBM_STORE_BF16R * 16 + 4: return launch_v2<LBM_STORE_BF16S, 4, true>(P, overlap, s);
     default: return dispatch<MODE_FUSED>(storage, flags & LBM_FLAG_EXACT, P, s);
   }
 }
@@ -513,7 +517,7 @@ int lbm_lattice_run_opts(const lbm_geometry* g, int32_t storage, void* pop_a, vo
     const bool last = s == nsteps - 1;
     P.rho_out = OutView{last ? rho_out : nullptr, 1, pitch, 0};
     P.u_out = OutView{last ? u_out : nullptr, 1, pitch, pitch * g->ny};
-    if (int e = launch_fused(storage, flags, P, (cudaStream_t)stream)) return e;
+    if (int e = launch_fused(storage, flags, P, s > 0, (cudaStream_t)stream)) return e;
   }
   if (counter != nullptr && nsteps > 0) {
     advance_counter_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(opt->step_counter, nsteps);

@@ -298,18 +298,18 @@ inline int launch_batch(const void* table, int n, int tiles, int bc_chunks, int*
   blocks = std::min(blocks, std::max(1, tiles));
   for (int k = 0; k < nsteps; ++k) {
     if (plain && tiles > 0) {
-      launch_step(batch_grid_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT>, dim3((unsigned)tiles), THREADS, k > 0, s, tab,
+      launch_step(batch_grid_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT>, dim3((unsigned)tiles), THREADS, k > 0, s, 0, tab,
                   start, n, (const int*)gbase, k);
       count_launch();
       if (int e = check_launch("batch_grid_kernel")) return e;
     } else {
-      launch_step(batch_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT>, dim3((unsigned)blocks), THREADS, k > 0, s, tab, start,
+      launch_step(batch_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT>, dim3((unsigned)blocks), THREADS, k > 0, s, 0, tab, start,
                   n, tiles, (const int*)gbase, k);
       count_launch();
       if (int e = check_launch("batch_kernel")) return e;
     }
     if (!HAS_BC && bc_chunks > 0) {
-      launch_step(batch_fixup_kernel<STORE, SHIFT>, dim3((unsigned)bc_chunks), kFixupChunk, true, s, tab, bc_start, n,
+      launch_step(batch_fixup_kernel<STORE, SHIFT>, dim3((unsigned)bc_chunks), kFixupChunk, true, s, 0, tab, bc_start, n,
                   (const int*)gbase, k);
       count_launch();
       if (int e = check_launch("batch_fixup_kernel")) return e;

@@ -316,33 +316,6 @@ __device__ __forceinline__ void collide_fast(R f[9], R rho, R ux, R uy, R omega)
 #undef LBM_PAIR
 }
 
-// The same collision on scaled deviations d_i = s (f_i - w_i) (float32): with
-// sd = s (rho - 1) = sum d_i and srho = s rho = s + sd,
-// d_i' = (1 - omega) d_i + omega w_i (sd + srho (4.5 cu^2 +- 3 cu - 1.5 |u|^2)).
-__device__ __forceinline__ void collide_dev(float d[9], float drho, float rho, float ux, float uy, float omega) {
-  const float om1 = 1.0f - omega;
-  const float Bd = -1.5f * fmaf(ux, ux, uy * uy);
-  const float orho = omega * rho, odr = omega * drho;
-  const float W0 = orho * wf(0), W1 = orho * wf(1), W5 = orho * wf(5);
-  const float D0 = odr * wf(0), D1 = odr * wf(1), D5 = odr * wf(5);
-  const float V1 = 3.0f * W1, V5 = 3.0f * W5;
-  d[0] = fmaf(om1, d[0], fmaf(W0, Bd, D0));
-  const float d58 = ux + uy, d67 = uy - ux;
-#define LBM_DPAIR(I, J, V, W, D, VV)                 \
-  {                                                 \
-    const float t = fmaf(4.5f * (V), (V), Bd);      \
-    const float s = fmaf((W), t, (D));              \
-    const float m = (VV) * (V);                     \
-    d[I] = fmaf(om1, d[I], s + m);                  \
-    d[J] = fmaf(om1, d[J], s - m);                  \
-  }
-  LBM_DPAIR(1, 3, ux, W1, D1, V1)
-  LBM_DPAIR(2, 4, uy, W1, D1, V1)
-  LBM_DPAIR(5, 7, d58, W5, D5, V5)
-  LBM_DPAIR(6, 8, d67, W5, D5, V5)
-#undef LBM_DPAIR
-}
-
 // ---- two nodes per instruction: packed float32 pairs (sm_100 family) --------
 __device__ __forceinline__ float2 f2c(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
@@ -358,7 +331,9 @@ __device__ __forceinline__ void moments9x2(const float2 f[9], float2& sum, float
   sum = add2(add2(add2(f[0], f[2]), add2(a, b)), f[4]);
 }
 
-// collide_dev on two nodes at once
+// The same collision on the scaled deviations d_i = s (f_i - w_i) (float32) of
+// two nodes: with sd = s (rho - 1) = sum d_i and srho = s rho = s + sd,
+// d_i' = (1 - omega) d_i + omega w_i (sd + srho (4.5 cu^2 +- 3 cu - 1.5 |u|^2)).
 __device__ __forceinline__ void collide_dev2(float2 d[9], float2 drho, float2 rho, float2 ux, float2 uy, float omega) {
   const float2 om1 = f2c(1.0f - omega), om = f2c(omega);
   const float2 Bd = mul2(f2c(-1.5f), fma2(ux, ux, mul2(uy, uy)));

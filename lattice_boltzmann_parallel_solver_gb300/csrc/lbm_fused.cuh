@@ -125,6 +125,56 @@ __device__ __forceinline__ void write_probe(const KParams& P, int x, int y, R ux
   }
 }
 
+// ---- one node's (or pair's) collision, shared by every fused body ---------------
+// fixed-point node: the integer collision, or float64 outside its range
+__device__ __forceinline__ void fx_collide_node(int64_t g[9], const fx::QConsts& qc, double omega) {
+  if (fx::collide_q(g, qc)) return;
+  double d[9];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) d[i] = fx::from_fx(g[i], wd(i));
+  const double r2 = density9(d);
+  double u2x, u2y;
+  velocity_fast(d, r2, u2x, u2y);
+  collide_fast(d, r2, u2x, u2y, omega);
+#pragma unroll
+  for (int i = 0; i < 9; ++i) g[i] = fx::to_fx(d[i], wd(i));
+}
+
+// float node on full populations
+template <typename R>
+__device__ __forceinline__ void collide_node(R g[9], R& rho, R& ux, R& uy, R omega) {
+  R jx, jy;
+  moments9(g, rho, jx, jy);
+  const R inv = rho != R(0) ? rcp_nr(rho) : R(0);
+  ux = jx * inv;
+  uy = jy * inv;
+  collide_fast(g, rho, ux, uy, omega);
+}
+
+// two nodes of a 16-bit storage, on the stored deviations (scale kS): rho is
+// s rho, sum is s (rho - 1)
+template <bool SHIFT>
+__device__ __forceinline__ void collide_pair(float2 g2[9], float2& sum, float2& rho, float2& ux, float2& uy,
+                                             float omega, float kS, const ShiftK& shk) {
+  float2 jx, jy;
+  moments9x2(g2, sum, jx, jy);
+  if constexpr (SHIFT) {
+    // the momentum of sig (its mass enters the collision through oS)
+    jx = add2(jx, f2c(shk.sx));
+    jy = add2(jy, f2c(shk.sy));
+  }
+  rho = add2(f2c(kS), sum);
+  const float2 inv = make_float2(rho.x != 0.0f ? rcp_nr(rho.x) : 0.0f, rho.y != 0.0f ? rcp_nr(rho.y) : 0.0f);
+  ux = mul2(jx, inv);
+  uy = mul2(jy, inv);
+  if constexpr (SHIFT) {
+    collide_dev2_ref(g2, sum, rho, ux, uy, omega, shk);
+    sum = add2(sum, f2c(shk.S));  // s (rho - 1) for the moments written out
+  } else {
+    collide_dev2(g2, sum, rho, ux, uy, omega);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Vectorised fused step.  Each thread owns NPT consecutive nodes of one row
 // (one aligned vector per population plane).  The six planes with cx = +-1
@@ -348,21 +398,8 @@ __device__ __forceinline__ void fused_v2_body(const KParams& P, const void* pop_
       float2 g2[9];
 #pragma unroll
       for (int i = 0; i < 9; ++i) g2[i] = make_float2(f[i][k], f[i][k1]);
-      float2 sum, jx, jy;
-      moments9x2(g2, sum, jx, jy);
-      if constexpr (SHIFT) {
-        // the momentum of sig (its mass enters the collision through oS)
-        jx = add2(jx, f2c(shk.sx));
-        jy = add2(jy, f2c(shk.sy));
-      }
-      const float2 rho = add2(f2c(kS), sum);  // s rho
-      const float2 inv = make_float2(rho.x != 0.0f ? rcp_nr(rho.x) : 0.0f, rho.y != 0.0f ? rcp_nr(rho.y) : 0.0f);
-      const float2 ux = mul2(jx, inv), uy = mul2(jy, inv);
-      if constexpr (SHIFT)
-        collide_dev2_ref(g2, sum, rho, ux, uy, omega, shk);
-      else
-        collide_dev2(g2, sum, rho, ux, uy, omega);
-      if constexpr (SHIFT) sum = add2(sum, f2c(shk.S));  // s (rho - 1) for the moments written out
+      float2 sum, rho, ux, uy;
+      collide_pair<SHIFT>(g2, sum, rho, ux, uy, omega, kS, shk);
       R ga[9], gb[9];
 #pragma unroll
       for (int i = 0; i < 9; ++i) {
@@ -380,16 +417,9 @@ __device__ __forceinline__ void fused_v2_body(const KParams& P, const void* pop_
       R g[9];
 #pragma unroll
       for (int i = 0; i < 9; ++i) g[i] = f[i][k];
-      R sum, jx, jy;
-      moments9(g, sum, jx, jy);
-      const R rho = SH ? kS + sum : sum;  // s rho for the 16-bit storages
-      const R inv = rho != R(0) ? rcp_nr(rho) : R(0);
-      const R ux = jx * inv, uy = jy * inv;
-      if constexpr (SH)
-        collide_dev(g, sum, rho, ux, uy, omega);
-      else
-        collide_fast(g, rho, ux, uy, omega);
-      node_extras(k, sum, rho, ux, uy, g);
+      R rho, ux, uy;
+      collide_node(g, rho, ux, uy, omega);
+      node_extras(k, rho, rho, ux, uy, g);
 #pragma unroll
       for (int i = 0; i < 9; ++i) f[i][k] = g[i];
     }
@@ -605,17 +635,7 @@ __device__ __forceinline__ void fused_fx_body(const KParams& P, const void* pop_
         write_probe(P, x, y, ux, uy, !HAS_BC, EDGES);
       }
     }
-    if (!fx::collide_q(g, P.qc)) {
-      double d[9];
-#pragma unroll
-      for (int i = 0; i < 9; ++i) d[i] = fx::from_fx(g[i], wd(i));
-      const double r2 = density9(d);
-      double u2x, u2y;
-      velocity_fast(d, r2, u2x, u2y);
-      collide_fast(d, r2, u2x, u2y, P.omega);
-#pragma unroll
-      for (int i = 0; i < 9; ++i) g[i] = fx::to_fx(d[i], wd(i));
-    }
+    fx_collide_node(g, P.qc, P.omega);
     if (pnode) {
       double br[9];
       bracket9_fast(ux, uy, br);
@@ -684,7 +704,7 @@ struct __align__(16) BatchEntry {
 // that one drains.  The first launch of a run stays a plain one: it may follow
 // any kernel of the caller's, also one that writes the geometry.
 template <typename... Params, typename... Args>
-inline void launch_step(void (*kernel)(Params...), dim3 grid, int threads, bool overlap, cudaStream_t s,
+inline void launch_step(void (*kernel)(Params...), dim3 grid, int threads, bool overlap, cudaStream_t s, size_t smem,
                         const Args&... args) {
   cudaLaunchAttribute at = {};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -692,6 +712,7 @@ inline void launch_step(void (*kernel)(Params...), dim3 grid, int threads, bool 
   cudaLaunchConfig_t c = {};
   c.gridDim = grid;
   c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
   c.stream = s;
   c.attrs = &at;
   c.numAttrs = overlap ? 1 : 0;

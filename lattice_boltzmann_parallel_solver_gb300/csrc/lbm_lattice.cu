@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "lbm_fused.cuh"
+#include "lbm_tile.h"
 
 namespace lbm {
 
@@ -281,13 +282,13 @@ constexpr int kV2Threads = 128;
   do {                                                                                 \
     const bool bc = P.g.bcmask != nullptr, pr = P.g.pressure != 0;                     \
     if (bc && pr)                                                                      \
-      launch_step(KERNEL<__VA_ARGS__, true, true>, grid, kV2Threads, overlap, s, P);   \
+      launch_step(KERNEL<__VA_ARGS__, true, true>, grid, kV2Threads, overlap, s, 0, P);   \
     else if (bc)                                                                       \
-      launch_step(KERNEL<__VA_ARGS__, true, false>, grid, kV2Threads, overlap, s, P);  \
+      launch_step(KERNEL<__VA_ARGS__, true, false>, grid, kV2Threads, overlap, s, 0, P);  \
     else if (pr)                                                                       \
-      launch_step(KERNEL<__VA_ARGS__, false, true>, grid, kV2Threads, overlap, s, P);  \
+      launch_step(KERNEL<__VA_ARGS__, false, true>, grid, kV2Threads, overlap, s, 0, P);  \
     else                                                                               \
-      launch_step(KERNEL<__VA_ARGS__, false, false>, grid, kV2Threads, overlap, s, P); \
+      launch_step(KERNEL<__VA_ARGS__, false, false>, grid, kV2Threads, overlap, s, 0, P); \
   } while (0)
 
 template <int NPT>
@@ -334,6 +335,19 @@ static int v2_npt(int storage, int flags, const KParams& P) {
   return npt;
 }
 
+// Lattices that may take several steps per launch: those of the vectorised
+// kernels at their default shape (a flag that picks a one-step kernel or where
+// the boundary sources go keeps the one-step launches).  Under the pressure
+// rewrite a tile's halo may hold columns 0 and nx-1 once per side only, and the
+// fixed-point storage stays with one step per launch: its rewrite runs in
+// float64, where each of a tile's warps pays for its one or two such nodes
+// (200x60: 9.8 us per step against 9.0).
+static bool tile_applies(int storage, int flags, const KParams& P) {
+  const int one_step = LBM_FLAG_EXACT | LBM_FLAG_GENERIC | LBM_FLAG_BC_INLINE | LBM_FLAG_BC_SPLIT | (15 << LBM_FLAG_NPT_SHIFT);
+  return (flags & one_step) == 0 && v2_fits(P, default_npt(storage)) &&
+         (!P.g.pressure || (P.g.nx >= 16 && storage != LBM_STORE_FX64));
+}
+
 constexpr int kFixupThreads = 128;
 
 template <int STORE, bool SHIFT = false>
@@ -341,9 +355,9 @@ template <int STORE, bool SHIFT = false>
 static int launch_fixup(const KParams& P, cudaStream_t s) {
   const dim3 grid((unsigned)((P.g.n_bcnodes + kFixupThreads - 1) / kFixupThreads));
   if (P.g.pressure)
-    launch_step(fixup_v2_kernel<STORE, kFixupThreads, true, SHIFT>, grid, kFixupThreads, true, s, P);
+    launch_step(fixup_v2_kernel<STORE, kFixupThreads, true, SHIFT>, grid, kFixupThreads, true, s, 0, P);
   else
-    launch_step(fixup_v2_kernel<STORE, kFixupThreads, false, SHIFT>, grid, kFixupThreads, true, s, P);
+    launch_step(fixup_v2_kernel<STORE, kFixupThreads, false, SHIFT>, grid, kFixupThreads, true, s, 0, P);
   count_launch();
   return check_launch("fixup_v2_kernel");
 }
@@ -506,18 +520,41 @@ int lbm_lattice_run_opts(const lbm_geometry* g, int32_t storage, void* pop_a, vo
   P.sr = (flags & LBM_FLAG_STOCHASTIC) != 0;
   P.qc = fx::q_consts(omega);
   P.step_dev = counter;
-  for (int s = 0; s < nsteps; ++s) {
-    // with a device counter the kernels hash (seed + s + *counter) themselves
-    P.seed = counter != nullptr ? seed + (uint32_t)s : hash32(seed + (uint32_t)s);
-    const bool even = (s % 2) == 0;
+  // small lattices take several steps per launch; the moments of the last step
+  // (rho_out, u_out) come from a one-step launch
+  P.pop_in = pop_a;
+  P.pop_out = pop_b;
+  P.aux_in = aux_a;
+  P.aux_out = aux_b;
+  const int tiled_steps = nsteps - (rho_out != nullptr || u_out != nullptr ? 1 : 0);
+  TilePlan plan;
+  if (tiled_steps >= 3 && tile_applies(storage, flags, P)) plan = tile_plan(storage, P);
+  if (plan.ksteps > 1)
+    if (int e = tile_prepare(storage, plan, P)) return e;
+  int launches = 0;
+  for (int s = 0; s < nsteps; ++launches) {
+    const bool even = (launches % 2) == 0;
     P.pop_in = even ? pop_a : pop_b;
     P.pop_out = even ? pop_b : pop_a;
     P.aux_in = even ? aux_a : aux_b;
     P.aux_out = even ? aux_b : aux_a;
+    // an odd number of steps per launch: the buffers alternate as they would
+    // step by step
+    const int left = tiled_steps - s;
+    const int k = plan.ksteps > 1 && left >= 3 ? std::min(plan.ksteps, left - (left % 2 == 0)) : 1;
+    if (k > 1) {
+      P.seed = seed + (uint32_t)s;
+      if (int e = tile_launch(storage, plan, k, P, s > 0, (cudaStream_t)stream)) return e;
+      s += k;
+      continue;
+    }
+    // with a device counter the kernels hash (seed + s + *counter) themselves
+    P.seed = counter != nullptr ? seed + (uint32_t)s : hash32(seed + (uint32_t)s);
     const bool last = s == nsteps - 1;
     P.rho_out = OutView{last ? rho_out : nullptr, 1, pitch, 0};
     P.u_out = OutView{last ? u_out : nullptr, 1, pitch, pitch * g->ny};
     if (int e = launch_fused(storage, flags, P, s > 0, (cudaStream_t)stream)) return e;
+    ++s;
   }
   if (counter != nullptr && nsteps > 0) {
     advance_counter_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(opt->step_counter, nsteps);

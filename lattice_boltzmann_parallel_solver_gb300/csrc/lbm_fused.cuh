@@ -20,6 +20,7 @@ struct GeoK {
   int pressure;
   uint32_t pin, pout;
   double rho_in, rho_out;
+  int64_t rho_in_q, rho_out_q;  // (rho - 1) 2^56
   int outlet;
   double kconst[LBM_MAX_SETS][9];
   double cconst[LBM_MAX_SETS][9];
@@ -138,6 +139,28 @@ __device__ __forceinline__ void fx_collide_node(int64_t g[9], const fx::QConsts&
   collide_fast(d, r2, u2x, u2y, omega);
 #pragma unroll
   for (int i = 0; i < 9; ++i) g[i] = fx::to_fx(d[i], wd(i));
+}
+
+// fixed-point node whose collision also feeds the pressure rewrite: g is
+// collided, pv the rewritten populations of the directions in `dirs`
+__device__ __forceinline__ void fx_pressure_node(int64_t g[9], int64_t pv[9], const KParams& P, bool inlet_side) {
+  const uint32_t dirs = inlet_side ? P.g.pin : P.g.pout;
+  if (fx::pressure_q(g, inlet_side ? P.g.rho_in_q : P.g.rho_out_q, dirs, pv)) {
+    fx_collide_node(g, P.qc, P.omega);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) pv[i] += g[i];
+    return;
+  }
+  double d[9], br[9], ux, uy;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) d[i] = fx::from_fx(g[i], wd(i));
+  const double rho = density9(d);
+  velocity_fast(d, rho, ux, uy);
+  bracket9_fast(ux, uy, br);
+  fx_collide_node(g, P.qc, P.omega);
+  const double rb = (inlet_side ? P.g.rho_in : P.g.rho_out) - rho;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) pv[i] = fx::to_fx(fma(wd(i) * br[i], rb, fx::from_fx(g[i], wd(i))), wd(i));
 }
 
 // float node on full populations
@@ -482,8 +505,8 @@ __device__ __forceinline__ void fused_v2_body(const KParams& P, const void* pop_
 // chunking, shuffles and boundary sources as fused_v2_body, on 64-bit integers:
 // pull, bounce-back and the outlet copy move populations exactly, the boundary
 // constants are rounded to fixed point, and fx::collide_q collides each node in
-// its range.  Nodes outside it, the moments written out (last step, probe) and
-// the pressure rewrite of columns 0 / nx-1 use float64 on the converted values.
+// its range.  Nodes outside it and the moments written out (last step, probe)
+// use float64 on the converted values.
 // The outlet memory holds the stored integers, as in the generic kernel.
 // ---------------------------------------------------------------------------
 template <int NPT, bool HAS_BC, bool HAS_PRESSURE, bool EDGES = false>
@@ -618,31 +641,29 @@ __device__ __forceinline__ void fused_fx_body(const KParams& P, const void* pop_
     const bool pnode = HAS_PRESSURE && P.g.pressure && k < nvalid && (x == nx - 2 || x == 1);
     const bool out = want_m && active && k < nvalid &&
                      (P.rho_out.p != nullptr || (P.probe_buf != nullptr && x == P.probe_x && y == P.probe_y));
-    double rho = 1.0, ux = 0.0, uy = 0.0;
-    if (out || pnode) {
+    if (out) {
       double d[9];
 #pragma unroll
       for (int i = 0; i < 9; ++i) d[i] = fx::from_fx(g[i], wd(i));
-      rho = density9(d);
+      const double rho = density9(d);
+      double ux, uy;
       velocity_fast(d, rho, ux, uy);
-      if (out) {
-        if (P.rho_out.p != nullptr) {
-          P.rho_out.p[x * P.rho_out.sx + y * P.rho_out.sy] = rho;
-          double* up = P.u_out.p + x * P.u_out.sx + y * P.u_out.sy;
-          up[0] = ux;
-          up[P.u_out.sc] = uy;
-        }
-        write_probe(P, x, y, ux, uy, !HAS_BC, EDGES);
+      if (P.rho_out.p != nullptr) {
+        P.rho_out.p[x * P.rho_out.sx + y * P.rho_out.sy] = rho;
+        double* up = P.u_out.p + x * P.u_out.sx + y * P.u_out.sy;
+        up[0] = ux;
+        up[P.u_out.sc] = uy;
       }
+      write_probe(P, x, y, ux, uy, !HAS_BC, EDGES);
     }
-    fx_collide_node(g, P.qc, P.omega);
     if (pnode) {
-      double br[9];
-      bracket9_fast(ux, uy, br);
-      const double rb = (x == nx - 2 ? P.g.rho_in : P.g.rho_out) - rho;
+      int64_t q[9];
+      fx_pressure_node(g, q, P, x == nx - 2);
 #pragma unroll
-      for (int i = 0; i < 9; ++i) pv[i] = fx::to_fx(fma(wd(i) * br[i], rb, fx::from_fx(g[i], wd(i))), wd(i));
+      for (int i = 0; i < 9; ++i) pv[i] = q[i];
       pcol = x;
+    } else {
+      fx_collide_node(g, P.qc, P.omega);
     }
 #pragma unroll
     for (int i = 0; i < 9; ++i) f[i][k] = g[i];
@@ -741,6 +762,8 @@ inline bool to_geok(const lbm_geometry* g, GeoK& k) {
   k.pout = g->pressure_out_dirs & 0x1FFu;
   k.rho_in = g->rho_in;
   k.rho_out = g->rho_out;
+  k.rho_in_q = fx::round_scaled(g->rho_in - 1.0, fx::kS);
+  k.rho_out_q = fx::round_scaled(g->rho_out - 1.0, fx::kS);
   k.outlet = g->outlet;
   std::memcpy(k.kconst, g->kconst, sizeof(k.kconst));
   std::memcpy(k.cconst, g->cconst, sizeof(k.cconst));

@@ -338,14 +338,10 @@ static int v2_npt(int storage, int flags, const KParams& P) {
 // Lattices that may take several steps per launch: those of the vectorised
 // kernels at their default shape (a flag that picks a one-step kernel or where
 // the boundary sources go keeps the one-step launches).  Under the pressure
-// rewrite a tile's halo may hold columns 0 and nx-1 once per side only, and the
-// fixed-point storage stays with one step per launch: its rewrite runs in
-// float64, where each of a tile's warps pays for its one or two such nodes
-// (200x60: 9.8 us per step against 9.0).
+// rewrite a tile's halo may hold columns 0 and nx-1 once per side only.
 static bool tile_applies(int storage, int flags, const KParams& P) {
   const int one_step = LBM_FLAG_EXACT | LBM_FLAG_GENERIC | LBM_FLAG_BC_INLINE | LBM_FLAG_BC_SPLIT | (15 << LBM_FLAG_NPT_SHIFT);
-  return (flags & one_step) == 0 && v2_fits(P, default_npt(storage)) &&
-         (!P.g.pressure || (P.g.nx >= 16 && storage != LBM_STORE_FX64));
+  return (flags & one_step) == 0 && v2_fits(P, default_npt(storage)) && (!P.g.pressure || P.g.nx >= 16);
 }
 
 constexpr int kFixupThreads = 128;

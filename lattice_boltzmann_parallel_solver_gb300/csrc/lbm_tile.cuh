@@ -350,25 +350,22 @@ __device__ __forceinline__ void tile_body(const KParams& P, const void* pop_in_v
         int64_t g[9];
 #pragma unroll
         for (int i = 0; i < 9; ++i) g[i] = f[i][0];
-        const bool pn = pressure_node(0), pb = probed(0);
-        double rho = 1.0, ux = 0.0, uy = 0.0;
-        if (pn || pb) {
-          double e[9];
+        if (probed(0)) {
+          double e[9], ux, uy;
 #pragma unroll
           for (int i = 0; i < 9; ++i) e[i] = fx::from_fx(g[i], wd(i));
-          rho = density9(e);
-          velocity_fast(e, rho, ux, uy);
-          if (pb) probe(0, ux, uy);
+          velocity_fast(e, density9(e), ux, uy);
+          probe(0, ux, uy);
         }
-        fx_collide_node(g, P.qc, P.omega);
-        if (pn) {
-          double br[9];
+        if (pressure_node(0)) {
+          int64_t q[9];
           V pv[9];
-          bracket9_fast(ux, uy, br);
-          const double rb = rho_target(0) - rho;
+          fx_pressure_node(g, q, P, xs[1] == nx - 2);
 #pragma unroll
-          for (int i = 0; i < 9; ++i) pv[i] = fx::to_fx(fma(wd(i) * br[i], rb, fx::from_fx(g[i], wd(i))), wd(i));
+          for (int i = 0; i < 9; ++i) pv[i] = q[i];
           rewrite(0, pv);
+        } else {
+          fx_collide_node(g, P.qc, P.omega);
         }
 #pragma unroll
         for (int i = 0; i < 9; ++i) f[i][0] = g[i];

@@ -66,12 +66,12 @@ typedef struct lbm_geometry {
   uint32_t pressure_in_dirs, pressure_out_dirs;
   double rho_in, rho_out;
   int32_t outlet; /* some node uses LBM_SRC_OUTLET */
-  /* device, the n_bcnodes linear indices y*nx + x (ascending) of the nodes with a
-   * bcmask bit.  With it, on lattices of at least 2^22 nodes in the 16-bit
-   * storages and 2^25 in the others (or with LBM_FLAG_BC_SPLIT), the vectorised
-   * step runs its boundary-free body over the whole lattice and then recomputes
-   * just these nodes with their sources; NULL, a smaller lattice or
-   * LBM_FLAG_BC_INLINE applies the sources inside the step. */
+  /* device, the n_bcnodes linear indices y*nx + x of the nodes with a bcmask
+   * bit.  With it, the vectorised step of the float32 storage, and of the others
+   * on lattices of at least 2^25 nodes (or with LBM_FLAG_BC_SPLIT), runs a
+   * boundary-free body over the lattice and recomputes just these nodes with
+   * their sources; NULL, a smaller lattice or LBM_FLAG_BC_INLINE applies the
+   * sources inside the step. */
   const int32_t* bcnodes;
   int32_t n_bcnodes;
   /* Plain inlet and outlet columns (all zero: none).  edge_inlet_desc is the
@@ -91,6 +91,17 @@ typedef struct lbm_geometry {
    * must give the same value.  The other storages do not use it (leave it 0);
    * every call checks that it lies inside (-0.5, 0.5). */
   double dev_ref_ux, dev_ref_uy;
+  /* The frame (0: not given; nx, ny >= 3).  Given, frame_desc holds the
+   * descriptors of row 0, row ny-1, column 0 and column nx-1 without their end
+   * nodes (0 for a row or column that only streams), then of the nodes (0, 0),
+   * (nx-1, 0), (0, ny-1) and (nx-1, ny-1), and every node with a bcmask bit that
+   * is not on the frame lies in columns inner_box[0]..inner_box[1] of rows
+   * inner_box[2]..inner_box[3] (none: inner_box[0] > inner_box[1]).  The
+   * vectorised steps then know a frame node's sources without reading the mask
+   * and the descriptor. */
+  int32_t frame;
+  uint32_t frame_desc[8];
+  int32_t inner_box[4];
 } lbm_geometry;
 
 /* ---- storage / arithmetic of the resident state ------------------------- */
@@ -286,13 +297,13 @@ size_t lbm_batch_table_bytes(int32_t n);
 /* Writes the device work table (table_bytes >= lbm_batch_table_bytes(n)) for
  * tiles of `rows` runs of `threads` threads x `npt` nodes; synchronises `stream`.
  * *bc_chunks receives the boundary-node plan that lbm_batch_run takes: -1 when
- * the boundary sources run inside the step (some lattice has boundary nodes
+ * the boundary sources run inside the tiles (some lattice has boundary nodes
  * but no list of them or sets LBM_FLAG_BC_INLINE, or the lattices hold fewer
- * than 2^20 nodes in total and none sets LBM_FLAG_BC_SPLIT: a second launch
- * per step would double the fixed cost of a small batch), else the number of
- * 128-node chunks of pass nodes: each step is then a boundary-free launch over
- * every node followed by a boundary-node pass over the chunks (bit-identical
- * results, fewer registers in the hot kernel). */
+ * than 2^17 nodes in total and none sets LBM_FLAG_BC_SPLIT), else a positive
+ * number that stands for the chunks of `threads` pass nodes: each step is then a
+ * boundary-free body over every node and a boundary-node pass over the chunks,
+ * in the same launch or, in the 16-bit storages from 2^20 nodes in total, in a
+ * second one (bit-identical results, fewer registers in the hot kernel). */
 int lbm_batch_build(const lbm_batch_lattice* lat, int32_t n, int32_t npt, int32_t threads, void* table,
                     size_t table_bytes, int32_t* total_tiles, int32_t* bc_chunks, void* stream);
 /* nsteps batched steps with `blocks` persistent blocks (0 = fill the GPU; more

@@ -49,6 +49,7 @@ class Geometry(C.Structure):
         ("bcnodes", vp), ("n_bcnodes", i32),
         ("edge_inlet_desc", C.c_uint32), ("edge_outlet_desc", C.c_uint32), ("n_bcnodes_edge", i32),
         ("dev_ref_ux", f64), ("dev_ref_uy", f64),
+        ("frame", i32), ("frame_desc", C.c_uint32 * 8), ("inner_box", i32 * 4),
     ]
 
 

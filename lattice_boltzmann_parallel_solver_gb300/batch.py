@@ -58,10 +58,11 @@ class Batch:
 
     def __init__(self, members=(), storage: str = "f16", npt: int = 0, threads: int = 0, blocks: int = None,
                  device: str = "cuda", stochastic: bool = None, rows: int = 0, inline_bc: bool | None = None):
-        """Batches of at least 2^20 nodes take each step as a boundary-free
-        launch over every node followed by a pass over the boundary nodes,
-        smaller ones as one launch with the boundary sources inside (same
-        results); ``inline_bc`` True / False forces the one or the other.
+        """Batches of at least 2^17 nodes (2^18 in the 16-bit storages) take each
+        step as a boundary-free body over every node and a pass over the
+        boundary nodes, in one launch (16-bit storages from 2^20 nodes: two),
+        smaller ones with the boundary sources inside the tiles (same results);
+        ``inline_bc`` True / False forces the one or the other.
         ``npt``, ``threads`` and ``rows`` (nodes per thread, threads per tile,
         runs of ``threads`` chunks per tile) default to what ``autotune`` picks
         for such batches (``_default_shape``; for large mixed von Karman
@@ -149,16 +150,23 @@ class Batch:
 
     # -- work table ----------------------------------------------------------------
     def _default_shape(self, nodes: int):
-        """Default nodes per thread / threads per tile: below 2^20 nodes (one
-        launch per step, boundary sources inside, row-segment tiles) 2 x 128
-        for the 16-bit storages and 1 x 128 for fx64; above (boundary-free step
-        over runs across row ends, then the boundary-node pass) 4 x 128 and
+        """Default nodes per thread / threads per tile: with the boundary sources
+        inside (row-segment tiles) 2 x 128 for the 16-bit storages and 1 x 128
+        for fx64; with the boundary-node pass (runs across row ends) 4 x 128 and
         1 x 64 (the reference-shifted 16-bit storages as the others)."""
-        split = self.inline_bc is False or (self.inline_bc is None and nodes >= (1 << 20))
+        split = not self._inline(nodes)
         if self._auto_shape[0]:
             self.npt = {"fx64": 1, "f64": 2}.get(self.storage, 4 if split or self.storage == "f32" else 2)
         if self._auto_shape[1]:
             self.threads = {"fx64": 64 if split else 128}.get(self.storage, 128)
+
+    def _inline(self, nodes: int) -> bool:
+        """Boundary sources inside the tiles: as asked, else below 2^17 nodes in
+        total (2^18 in the 16-bit storages, whose tiles pay more for leaving the
+        boundary nodes out)."""
+        if self.inline_bc is not None:
+            return self.inline_bc
+        return nodes < (1 << (18 if self.storage in SIXTEEN_BIT else 17))
 
     def _rows(self) -> int:
         """Runs per tile (a run: ``threads`` consecutive chunks of ``npt``
@@ -194,7 +202,7 @@ class Batch:
                 c.probe_x = c.probe_y = -1
             c.seed = int(m.seed) & 0xFFFFFFFF
             c.flags = (_lib.FLAG_STOCHASTIC if self.stochastic else 0) | \
-                {True: _lib.FLAG_BC_INLINE, False: _lib.FLAG_BC_SPLIT}.get(self.inline_bc, 0)
+                (_lib.FLAG_BC_INLINE if self._inline(self.nodes) else _lib.FLAG_BC_SPLIT if self.inline_bc is False else 0)
             c.rows = rows
         size = int(_lib.load().lbm_batch_table_bytes(n))
         self.table = torch.empty(size, dtype=torch.uint8, device=self.device)

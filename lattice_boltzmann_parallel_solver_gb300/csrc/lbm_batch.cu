@@ -10,7 +10,7 @@ using namespace lbm;
 extern "C" {
 
 size_t lbm_batch_table_bytes(int32_t n) {
-  return (size_t)n * sizeof(BatchEntry) + 2 * (size_t)n * sizeof(int) + 256;
+  return 2 * (size_t)n * sizeof(BatchEntry) + 2 * (size_t)n * sizeof(int) + 256;
 }
 
 int lbm_batch_build(const lbm_batch_lattice* lat, int32_t n, int32_t npt, int32_t threads, void* table,
@@ -67,10 +67,9 @@ int lbm_batch_build(const lbm_batch_lattice* lat, int32_t n, int32_t npt, int32_
     if (L.flags & LBM_FLAG_BC_SPLIT) force_split = true;
     nodes += (int64_t)L.g->nx * L.g->ny;
     bc_start[(size_t)j] = (int)chunks_bc;
-    chunks_bc += (pass_nodes(e.P.g) + kFixupChunk - 1) / kFixupChunk;
+    chunks_bc += (pass_nodes(e.P.g) + threads - 1) / threads;
   }
-  // small batches keep one launch per step (the pass would double their fixed cost)
-  if (nodes < kBatchSplitNodes && !force_split) inline_bc = true;
+  if (nodes < kBatchPassNodes && !force_split) inline_bc = true;
   // tiles: runs across row ends with the pass, row segments without it
   for (int j = 0; j < n; ++j) {
     const BatchEntry& e = ent[(size_t)j];
@@ -82,8 +81,13 @@ int lbm_batch_build(const lbm_batch_lattice* lat, int32_t n, int32_t npt, int32_
       tiles += ((int64_t)e.cpr * e.P.g.ny + run - 1) / run;
     }
   }
-  if (tiles >= ((int64_t)1 << 31) || chunks_bc >= ((int64_t)1 << 31))
+  if (tiles + chunks_bc >= ((int64_t)1 << 31) || chunks_bc >= kPlanMerged)
     return set_error(LBM_ERR_ARG, "too many tiles");
+  // a second copy of the entries for the fixed-point kernels
+  for (int j = 0; j < n; ++j) {
+    ent.push_back(ent[(size_t)j]);
+    set_fx_tables(ent.back().P.g);
+  }
   char* dst = static_cast<char*>(table);
   const size_t eb = ent.size() * sizeof(BatchEntry), ib = (size_t)n * sizeof(int);
   cudaError_t err = cudaMemcpyAsync(dst, ent.data(), eb, cudaMemcpyHostToDevice, (cudaStream_t)stream);
@@ -94,7 +98,7 @@ int lbm_batch_build(const lbm_batch_lattice* lat, int32_t n, int32_t npt, int32_
   if (err == cudaSuccess) err = cudaStreamSynchronize((cudaStream_t)stream);
   if (err != cudaSuccess) return set_error(LBM_ERR_CUDA, cudaGetErrorString(err));
   *total_tiles = (int32_t)tiles;
-  *bc_chunks = inline_bc ? -1 : (int32_t)chunks_bc;
+  *bc_chunks = inline_bc ? -1 : (int32_t)chunks_bc | (nodes < kBatchSplitNodes ? kPlanMerged : 0);
   return LBM_OK;
 }
 

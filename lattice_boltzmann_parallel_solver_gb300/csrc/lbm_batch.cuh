@@ -65,7 +65,7 @@ __device__ __forceinline__ int owner_of(const int* __restrict__ start, int n, in
 
 // One tile of lattice `e` (staged in shared memory) at global step g; SHIFT:
 // the reference-shifted 16-bit storages.
-template <int STORE, int NPT, int THREADS, bool HAS_BC, bool SHIFT>
+template <int STORE, int NPT, int THREADS, bool HAS_BC, bool SHIFT, bool MERGED>
 __device__ __forceinline__ void batch_tile(const BatchEntry& e, int local, int g) {
   const bool odd = (g - e.s0) & 1;
   const void* pin = odd ? e.pop_b : e.pop_a;
@@ -79,13 +79,13 @@ __device__ __forceinline__ void batch_tile(const BatchEntry& e, int local, int g
   const bool pressure = HAS_BC && e.P.g.pressure != 0;
   // the boundary-free body applies the plain inlet / outlet columns itself
   // (EDGES), the boundary-node pass the other boundary nodes
-  auto step_chunk = [&](int x0, int y) {
+  auto step_chunk = [&](int x0, int y, bool special) {
     if constexpr (STORE == LBM_STORE_FX64) {
-      if (pressure) fused_fx_body<NPT, HAS_BC, HAS_BC, !HAS_BC>(e.P, pin, pout, ain, aout, x0, y);
-      else fused_fx_body<NPT, HAS_BC, false, !HAS_BC>(e.P, pin, pout, ain, aout, x0, y);
+      if (pressure) fused_fx_body<NPT, HAS_BC, HAS_BC, !HAS_BC, MERGED>(e.P, pin, pout, ain, aout, x0, y, special);
+      else fused_fx_body<NPT, HAS_BC, false, !HAS_BC, MERGED>(e.P, pin, pout, ain, aout, x0, y, special);
     } else {
-      if (pressure) fused_v2_body<STORE, NPT, HAS_BC, HAS_BC, !HAS_BC, SHIFT>(e.P, pin, pout, ain, aout, x0, y, seed);
-      else fused_v2_body<STORE, NPT, HAS_BC, false, !HAS_BC, SHIFT>(e.P, pin, pout, ain, aout, x0, y, seed);
+      if (pressure) fused_v2_body<STORE, NPT, HAS_BC, HAS_BC, !HAS_BC, SHIFT, MERGED>(e.P, pin, pout, ain, aout, x0, y, seed, false, special);
+      else fused_v2_body<STORE, NPT, HAS_BC, false, !HAS_BC, SHIFT, MERGED>(e.P, pin, pout, ain, aout, x0, y, seed, false, special);
     }
   };
   if constexpr (HAS_BC) {
@@ -96,7 +96,7 @@ __device__ __forceinline__ void batch_tile(const BatchEntry& e, int local, int g
     const int yb = local / e.xblocks, xb = local - yb * e.xblocks;
     const int x0 = (xb * THREADS + (int)threadIdx.x) * NPT;
     const int y1 = min((yb + 1) * e.rows, e.P.g.ny);
-    for (int y = yb * e.rows; y < y1; ++y) step_chunk(x0, y);
+    for (int y = yb * e.rows; y < y1; ++y) step_chunk(x0, y, false);
   } else {
     // runs of THREADS consecutive chunks, chunks numbered row by row: no
     // idle lanes at row ends.  The lanes of a run past the lattice's last
@@ -116,55 +116,17 @@ __device__ __forceinline__ void batch_tile(const BatchEntry& e, int local, int g
         y = e.P.g.ny - 1;
         x0 = e.P.g.nx;
       }
-      step_chunk(x0, y);
+      bool special = false;
+      if constexpr (MERGED) {
+        // the warp's chunks: 32 in a row from its first one, or some row end
+        const int xa = __shfl_sync(0xffffffffu, x0, 0), ya = __shfl_sync(0xffffffffu, y, 0);
+        special = pass_chunk(e.P.g, xa, 32 * NPT, ya);
+      }
+      step_chunk(x0, y, special);
     }
   }
 }
 
-// The persistent form: block b walks the contiguous span of tiles
-// [b T / B, (b + 1) T / B) (T tiles, B blocks), so consecutive tiles mostly
-// belong to one lattice: the owner search and the entry staging happen once per
-// lattice the span touches, not once per tile, and the spans differ by at most
-// one tile (no tail of partly filled waves).
-template <int STORE, int NPT, int THREADS, bool HAS_BC, bool SHIFT>
-__global__ void __launch_bounds__(THREADS, batch_min_blocks<STORE, NPT, THREADS, HAS_BC>())
-    batch_kernel(const BatchEntry* __restrict__ tab, const int* __restrict__ tile_start, int n_inst,
-                 int total_tiles, const int* __restrict__ gbase, int k) {
-  // the current lattice's entry, staged in shared memory: the body reads its
-  // parameters many times per tile, and in global memory the streaming
-  // population traffic would evict them from L1
-  __shared__ __align__(16) unsigned char ebuf[sizeof(BatchEntry)];
-  const BatchEntry& e = *reinterpret_cast<const BatchEntry*>(ebuf);
-  const int per = total_tiles / (int)gridDim.x, extra = total_tiles % (int)gridDim.x;
-  const int b = (int)blockIdx.x;
-  const int t0 = b * per + min(b, extra), t1 = t0 + per + (b < extra ? 1 : 0);
-  if (t0 >= t1) {
-    pdl_wait();
-    return;
-  }
-  const int g = *gbase + k;
-  int lo = owner_of(tile_start, n_inst, t0);
-  int first = __ldg(tile_start + lo);
-  int next = lo + 1 < n_inst ? __ldg(tile_start + lo + 1) : total_tiles;
-  stage_entry<THREADS, HAS_BC>(tab, lo, ebuf);
-  pdl_wait();  // the table and the global step are not written during a run
-  for (int tile = t0; tile < t1; ++tile) {
-    if (tile >= next) {
-      do {
-        ++lo;
-        first = next;
-        next = lo + 1 < n_inst ? __ldg(tile_start + lo + 1) : total_tiles;
-      } while (tile >= next);
-      stage_entry<THREADS, HAS_BC>(tab, lo, ebuf);
-    }
-    if (g >= e.s0 && g < e.s_end) batch_tile<STORE, NPT, THREADS, HAS_BC, SHIFT>(e, tile - first, g);
-  }
-}
-
-// The plain-grid form (one tile per block, block b = tile b).  The block
-// copies the lattices' tile starts into shared memory (one round trip) and
-// finds its lattice there, instead of a search through global memory (a
-// dependent L2 round trip per halving).
 constexpr int kStartSmem = 512;
 
 // owner_of for a whole block: the start list is copied into shared memory
@@ -184,55 +146,45 @@ __device__ __forceinline__ int owner_of_staged(const int* __restrict__ start, in
   return a;
 }
 
-template <int STORE, int NPT, int THREADS, bool HAS_BC, bool SHIFT>
-__global__ void __launch_bounds__(THREADS, batch_min_blocks<STORE, NPT, THREADS, HAS_BC>())
-    batch_grid_kernel(const BatchEntry* __restrict__ tab, const int* __restrict__ tile_start, int n_inst,
-                      const int* __restrict__ gbase, int k) {
-  __shared__ __align__(16) unsigned char ebuf[sizeof(BatchEntry)];
-  const BatchEntry& e = *reinterpret_cast<const BatchEntry*>(ebuf);
-  const int tile = (int)blockIdx.x;
-  const int lo = owner_of_staged<THREADS>(tile_start, n_inst, tile);
-  stage_entry<THREADS, HAS_BC>(tab, lo, ebuf);
-  const int g = *gbase + k;
-  pdl_wait();  // the table and the global step are not written during a run
-  if (g < e.s0 || g >= e.s_end) return;
-  batch_tile<STORE, NPT, THREADS, HAS_BC, SHIFT>(e, tile - __ldg(tile_start + lo), g);
-}
+// The boundary-node pass of a batch, in the first bc_chunks blocks of a launch
+// whose other blocks leave the pass nodes out (MERGED), or in a second launch
+// that overwrites their outputs.  One thread per pass node recomputes that node
+// with its sources and, under the pressure rewrite, with the rewrite (the body at
+// one node per thread, the same arithmetic and random bits as the in-step
+// sources).  A lattice's pass nodes are its listed
+// boundary nodes other than the plain edge nodes (the boundary-free body applies
+// those itself), then, under the pressure rewrite, columns 1 and nx-2 of every
+// row (those not listed already), whose nodes write the rewritten populations of
+// columns nx-1 and 0.  Block b takes chunk b of the chunk list: lattice j owns
+// chunks [bc_start[j], bc_start[j + 1]) of THREADS pass nodes.
 
-// The batched boundary-node pass: after batch_kernel<..., false> stepped every
-// node of every live lattice without boundary sources or pressure rewrite
-// (but with the plain inlet / outlet columns), one thread per pass node
-// recomputes that node with them and overwrites its outputs (the body at one
-// node per thread, the same arithmetic and random bits as the in-step
-// sources).  A lattice's pass nodes are its listed boundary nodes other than
-// the plain edge nodes, then, under the pressure rewrite, columns 1 and nx-2 of
-// every row (those not listed already), whose nodes write the rewritten
-// populations of columns nx-1 and 0.  Block b takes chunk b of the chunk list: lattice j owns
-// chunks [bc_start[j], bc_start[j + 1]) of kFixupChunk pass nodes.
-constexpr int kFixupChunk = 128;
-
-// batches below this many nodes in total keep the sources inside one launch
-// per step (a second launch per step would double a small batch's fixed cost)
-constexpr int64_t kBatchSplitNodes = (int64_t)1 << 20;
+// Where a batch applies its boundary sources, by its nodes in total (us per
+// step, inside the tiles / pass in the same launch / pass as a second launch):
+//   below kBatchPassNodes inside the tiles (six 108x110 channels and the like; a
+//     caller with 16-bit storages asks for it up to 2^18: 151k nodes 5.7 / 6.0)
+//   from there in the same launch: six 420x180 channels fx64 21.0 / 17.3 / 24.6,
+//     f16 11.6 / 8.9 / 9.8; 1.0M nodes fx64 42.4 / 34.5 / 42.4, f16 19.2 / 13.4 / 14.8
+//   from kBatchSplitNodes the 16-bit storages take the second launch, whose main
+//     body is free of the pass's tests: 1.5M nodes f16 31.3 / 22.5 / 19.8, 4.8M 72 /
+//     55 / 50; the other storages stay (1.5M nodes fx64 60.3 / 50.0 / 57.5)
+constexpr int64_t kBatchPassNodes = (int64_t)1 << 17, kBatchSplitNodes = (int64_t)1 << 20;
+// set in the plan of a batch below kBatchSplitNodes
+constexpr int kPlanMerged = 1 << 30;
 
 inline int64_t pass_nodes(const GeoK& g) {
   return (g.bcmask != nullptr ? (int64_t)(g.n_bcnodes - g.n_bcnodes_edge) : 0) + (g.pressure ? 2 * (int64_t)g.ny : 0);
 }
 
-// 64 registers: 8 blocks of the latency-bound pass per SM (f16 takes 66
-// without the cap, 7 blocks); the fixed-point body would spill under it
-template <int STORE, bool SHIFT>
-__global__ void __launch_bounds__(kFixupChunk, STORE == LBM_STORE_FX64 ? 1 : 8)
-    batch_fixup_kernel(const BatchEntry* __restrict__ tab, const int* __restrict__ bc_start, int n_inst,
-                       const int* __restrict__ gbase, int k) {
-  __shared__ __align__(16) unsigned char ebuf[sizeof(BatchEntry)];
+template <int STORE, int THREADS, bool SHIFT>
+__device__ __forceinline__ void batch_pass(const BatchEntry* __restrict__ tab, const int* __restrict__ bc_start,
+                                           int n_inst, const int* __restrict__ gbase, int k, unsigned char* ebuf) {
   const BatchEntry& e = *reinterpret_cast<const BatchEntry*>(ebuf);
   const int g = *gbase + k;
-  const int j = owner_of_staged<kFixupChunk>(bc_start, n_inst, (int)blockIdx.x);
-  stage_entry<kFixupChunk, true>(tab, j, ebuf);
-  pdl_wait();
+  const int j = owner_of_staged<THREADS>(bc_start, n_inst, (int)blockIdx.x);
+  stage_entry<THREADS, true>(tab, j, ebuf);
+  pdl_wait();  // the table and the global step are not written during a run
   if (g < e.s0 || g >= e.s_end) return;
-  const int t = ((int)blockIdx.x - __ldg(bc_start + j)) * kFixupChunk + (int)threadIdx.x;
+  const int t = ((int)blockIdx.x - __ldg(bc_start + j)) * THREADS + (int)threadIdx.x;
   const int nx = e.P.g.nx;
   const int listed = e.P.g.bcmask != nullptr ? e.P.g.n_bcnodes - e.P.g.n_bcnodes_edge : 0;
   int x, y;
@@ -269,14 +221,91 @@ __global__ void __launch_bounds__(kFixupChunk, STORE == LBM_STORE_FX64 ? 1 : 8)
   }
 }
 
+// The persistent form: block b walks the contiguous span of tiles
+// [b T / B, (b + 1) T / B) (T tiles, B blocks), so consecutive tiles mostly
+// belong to one lattice: the owner search and the entry staging happen once per
+// lattice the span touches, not once per tile, and the spans differ by at most
+// one tile (no tail of partly filled waves).
+template <int STORE, int NPT, int THREADS, bool HAS_BC, bool SHIFT, bool MERGED>
+__global__ void __launch_bounds__(THREADS, batch_min_blocks<STORE, NPT, THREADS, HAS_BC>())
+    batch_kernel(const BatchEntry* __restrict__ tab, const int* __restrict__ tile_start, int n_inst,
+                 int total_tiles, const int* __restrict__ bc_start, int bc_chunks, const int* __restrict__ gbase,
+                 int k) {
+  // the current lattice's entry, staged in shared memory: the body reads its
+  // parameters many times per tile, and in global memory the streaming
+  // population traffic would evict them from L1
+  __shared__ __align__(16) unsigned char ebuf[sizeof(BatchEntry)];
+  const BatchEntry& e = *reinterpret_cast<const BatchEntry*>(ebuf);
+  if (MERGED && (int)blockIdx.x < bc_chunks) {
+    batch_pass<STORE, THREADS, SHIFT>(tab, bc_start, n_inst, gbase, k, ebuf);
+    return;
+  }
+  const int blocks = (int)gridDim.x - bc_chunks, b = (int)blockIdx.x - bc_chunks;
+  const int per = total_tiles / blocks, extra = total_tiles % blocks;
+  const int t0 = b * per + min(b, extra), t1 = t0 + per + (b < extra ? 1 : 0);
+  if (t0 >= t1) {
+    pdl_wait();
+    return;
+  }
+  const int g = *gbase + k;
+  int lo = owner_of(tile_start, n_inst, t0);
+  int first = __ldg(tile_start + lo);
+  int next = lo + 1 < n_inst ? __ldg(tile_start + lo + 1) : total_tiles;
+  stage_entry<THREADS, HAS_BC>(tab, lo, ebuf);
+  pdl_wait();  // the table and the global step are not written during a run
+  for (int tile = t0; tile < t1; ++tile) {
+    if (tile >= next) {
+      do {
+        ++lo;
+        first = next;
+        next = lo + 1 < n_inst ? __ldg(tile_start + lo + 1) : total_tiles;
+      } while (tile >= next);
+      stage_entry<THREADS, HAS_BC>(tab, lo, ebuf);
+    }
+    if (g >= e.s0 && g < e.s_end) batch_tile<STORE, NPT, THREADS, HAS_BC, SHIFT, MERGED>(e, tile - first, g);
+  }
+}
+
+// The plain-grid form (one tile per block).  The block copies the lattices' tile
+// starts into shared memory (one round trip) and finds its lattice there, instead
+// of a search through global memory (a dependent L2 round trip per halving).
+template <int STORE, int NPT, int THREADS, bool HAS_BC, bool SHIFT, bool MERGED>
+__global__ void __launch_bounds__(THREADS, batch_min_blocks<STORE, NPT, THREADS, HAS_BC>())
+    batch_grid_kernel(const BatchEntry* __restrict__ tab, const int* __restrict__ tile_start, int n_inst,
+                      const int* __restrict__ bc_start, int bc_chunks, const int* __restrict__ gbase, int k) {
+  __shared__ __align__(16) unsigned char ebuf[sizeof(BatchEntry)];
+  const BatchEntry& e = *reinterpret_cast<const BatchEntry*>(ebuf);
+  if (MERGED && (int)blockIdx.x < bc_chunks) {
+    batch_pass<STORE, THREADS, SHIFT>(tab, bc_start, n_inst, gbase, k, ebuf);
+    return;
+  }
+  const int tile = (int)blockIdx.x - bc_chunks;
+  const int lo = owner_of_staged<THREADS>(tile_start, n_inst, tile);
+  stage_entry<THREADS, HAS_BC>(tab, lo, ebuf);
+  const int g = *gbase + k;
+  pdl_wait();  // the table and the global step are not written during a run
+  if (g < e.s0 || g >= e.s_end) return;
+  batch_tile<STORE, NPT, THREADS, HAS_BC, SHIFT, MERGED>(e, tile - __ldg(tile_start + lo), g);
+}
+
+// the pass as a launch of its own
+template <int STORE, int THREADS, bool SHIFT>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
+    batch_fixup_kernel(const BatchEntry* __restrict__ tab, const int* __restrict__ bc_start, int n_inst,
+                       const int* __restrict__ gbase, int k) {
+  __shared__ __align__(16) unsigned char ebuf[sizeof(BatchEntry)];
+  batch_pass<STORE, THREADS, SHIFT>(tab, bc_start, n_inst, gbase, k, ebuf);
+}
+
 // one copy per translation unit (each unit launches its own)
 static __global__ void batch_advance_kernel(int* gbase, int k) { *gbase += k; }
 
-template <int STORE, int NPT, int THREADS, bool HAS_BC, bool SHIFT = false>
-inline int launch_batch(const void* table, int n, int tiles, int bc_chunks, int* gbase, int nsteps, int blocks,
+template <int STORE, int NPT, int THREADS, bool HAS_BC, bool SHIFT, bool MERGED>
+inline int launch_batch_form(const void* table, int n, int tiles, int bc_chunks, int* gbase, int nsteps, int blocks,
                         cudaStream_t s) {
-  const BatchEntry* tab = static_cast<const BatchEntry*>(table);
-  const int* start = reinterpret_cast<const int*>(static_cast<const char*>(table) + (size_t)n * sizeof(BatchEntry));
+  // the entries with float64 boundary constants, then with fixed-point ones
+  const BatchEntry* tab = static_cast<const BatchEntry*>(table) + (STORE == LBM_STORE_FX64 ? n : 0);
+  const int* start = reinterpret_cast<const int*>(static_cast<const char*>(table) + 2 * (size_t)n * sizeof(BatchEntry));
   const int* bc_start = start + n;
   if (blocks <= 0) {
     // resident blocks of this kernel on the whole GPU, queried on the first
@@ -286,7 +315,7 @@ inline int launch_batch(const void* table, int n, int tiles, int bc_chunks, int*
       int per_sm = 0, sms = 0, dev = 0;
       cudaGetDevice(&dev);
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT>,
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT, MERGED>,
                                                     THREADS, 0);
       fill = std::max(1, sms * std::max(1, per_sm));
     }
@@ -296,21 +325,22 @@ inline int launch_batch(const void* table, int n, int tiles, int bc_chunks, int*
   // block; otherwise persistent blocks walk contiguous spans of tiles
   const bool plain = (int64_t)blocks * 2 > (int64_t)tiles;
   blocks = std::min(blocks, std::max(1, tiles));
+  const int pass = MERGED ? bc_chunks : 0;
   for (int k = 0; k < nsteps; ++k) {
     if (plain && tiles > 0) {
-      launch_step(batch_grid_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT>, dim3((unsigned)tiles), THREADS, k > 0, s, 0, tab,
-                  start, n, (const int*)gbase, k);
+      launch_step(batch_grid_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT, MERGED>, dim3((unsigned)(pass + tiles)), THREADS, k > 0,
+                  s, 0, tab, start, n, bc_start, pass, (const int*)gbase, k);
       count_launch();
       if (int e = check_launch("batch_grid_kernel")) return e;
     } else {
-      launch_step(batch_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT>, dim3((unsigned)blocks), THREADS, k > 0, s, 0, tab, start,
-                  n, tiles, (const int*)gbase, k);
+      launch_step(batch_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT, MERGED>, dim3((unsigned)(pass + blocks)), THREADS, k > 0, s, 0,
+                  tab, start, n, tiles, bc_start, pass, (const int*)gbase, k);
       count_launch();
       if (int e = check_launch("batch_kernel")) return e;
     }
-    if (!HAS_BC && bc_chunks > 0) {
-      launch_step(batch_fixup_kernel<STORE, SHIFT>, dim3((unsigned)bc_chunks), kFixupChunk, true, s, 0, tab, bc_start, n,
-                  (const int*)gbase, k);
+    if (!HAS_BC && !MERGED && bc_chunks > 0) {
+      launch_step(batch_fixup_kernel<STORE, THREADS, SHIFT>, dim3((unsigned)bc_chunks), THREADS, true, s, 0, tab, bc_start,
+                  n, (const int*)gbase, k);
       count_launch();
       if (int e = check_launch("batch_fixup_kernel")) return e;
     }
@@ -320,6 +350,20 @@ inline int launch_batch(const void* table, int n, int tiles, int bc_chunks, int*
   return check_launch("batch_advance_kernel");
 }
 
+
+template <int STORE, int NPT, int THREADS, bool HAS_BC, bool SHIFT = false>
+inline int launch_batch(const void* table, int n, int tiles, int bc_chunks, int* gbase, int nsteps, int blocks,
+                        cudaStream_t s) {
+  if constexpr (HAS_BC) {
+    return launch_batch_form<STORE, NPT, THREADS, true, SHIFT, false>(table, n, tiles, 0, gbase, nsteps, blocks, s);
+  } else {
+    const int chunks = bc_chunks & ~kPlanMerged;
+    if constexpr (Store<STORE>::kShifted)
+      if (!(bc_chunks & kPlanMerged))
+        return launch_batch_form<STORE, NPT, THREADS, false, SHIFT, false>(table, n, tiles, chunks, gbase, nsteps, blocks, s);
+    return launch_batch_form<STORE, NPT, THREADS, false, SHIFT, true>(table, n, tiles, chunks, gbase, nsteps, blocks, s);
+  }
+}
 
 // dispatch over (storage, npt, threads) to launch_batch<..., HAS_BC>
 int batch_launch_inline(const void* table, int n, int tiles, int bc_chunks, int storage, int npt, int threads,

@@ -32,7 +32,12 @@ struct GeoK {
   double edge_in_f[9];
   // reference velocity of the reference-shifted 16-bit storages
   double dev_ref_ux, dev_ref_uy;
+  // the frame's descriptors (lbm_geometry; all 0 when it is not given) and the
+  // box of the other boundary nodes (the whole lattice when it is not given)
+  uint32_t frame_desc[8];
+  int box_x0, box_x1, box_y0, box_y1;
 };
+
 
 struct View {
   const double* p;
@@ -77,6 +82,8 @@ struct KParams {
   int dev_shift;
   // fixed-point storage: constants of its collision
   fx::QConsts qc;
+  // rows of blocks at the start of the grid that recompute the boundary nodes
+  int pass_rows;
 };
 
 // Programmatic dependent launch.  A step's kernel that was launched with the
@@ -106,14 +113,15 @@ __device__ __forceinline__ bool plain_edge_node(const KParams& P, int x, int y) 
 }
 
 // skip_bc: a body without its boundary block leaves the probe of a node that
-// the batched boundary-node pass recomputes (a listed boundary node other than
-// the plain edge nodes the body applies itself when ``edges`` is set, or,
-// under the pressure rewrite, a node of column 1 or nx-2) to that pass
+// the boundary-node pass recomputes (a listed boundary node other than the plain
+// edge nodes the body applies itself when ``edges`` is set, or, when the pass
+// also does the pressure rewrite (pass_pressure), a node of column 1 or nx-2) to
+// that pass
 template <typename R>
 __device__ __forceinline__ void write_probe(const KParams& P, int x, int y, R ux, R uy, bool skip_bc = false,
-                                            bool edges = false) {
+                                            bool edges = false, bool pass_pressure = false) {
   if (P.probe_buf != nullptr && x == P.probe_x && y == P.probe_y) {
-    if (skip_bc && ((P.g.pressure && (x == 1 || x == P.g.nx - 2)) ||
+    if (skip_bc && ((pass_pressure && P.g.pressure && (x == 1 || x == P.g.nx - 2)) ||
                     (P.g.bcmask != nullptr && ((__ldg(P.g.bcmask + y * P.g.words + (x >> 5)) >> (x & 31)) & 1u) &&
                      !(edges && plain_edge_node(P, x, y)))))
       return;
@@ -124,6 +132,49 @@ __device__ __forceinline__ void write_probe(const KParams& P, int x, int y, R ux
     }
     *P.probe_count = t + 1;
   }
+}
+
+// descriptor of a node on the frame, 0 inside it
+__device__ __forceinline__ uint32_t frame_desc(const GeoK& g, int x, int y) {
+  const bool left = x == 0, right = x == g.nx - 1;
+  if (y == 0) return left ? g.frame_desc[4] : (right ? g.frame_desc[5] : g.frame_desc[0]);
+  if (y == g.ny - 1) return left ? g.frame_desc[6] : (right ? g.frame_desc[7] : g.frame_desc[1]);
+  return left ? g.frame_desc[2] : (right ? g.frame_desc[3] : 0u);
+}
+
+// Whether columns [xa, xb] of row y (a warp's) are inside: no periodic wrap, no
+// outlet memory, no pressure column, and (bc) no boundary node.
+__device__ __forceinline__ bool inside(const GeoK& g, bool bc, int xa, int xb, int y) {
+  if (xa < 2 || xb > g.nx - 3 || y < 1 || y > g.ny - 2) return false;
+  return !bc || y < g.box_y0 || y > g.box_y1 || xb < g.box_x0 || xa > g.box_x1;
+}
+
+// Whether columns [x0, x0 + npt) of row y may hold nodes of the boundary-node pass
+// (or, under the pressure rewrite, of columns 0, 1, nx-2, nx-1): the ``special``
+// argument of the bodies that leave those out, for a block's or a warp's columns,
+// so that the test costs the other warps' lanes nothing
+__device__ __forceinline__ bool pass_chunk(const GeoK& g, int x0, int npt, int y) {
+  return y == 0 || y == g.ny - 1 || x0 < 2 || x0 + npt >= g.nx - 1 ||
+         (y >= g.box_y0 && y <= g.box_y1 && x0 + npt > g.box_x0 && x0 <= g.box_x1);
+}
+
+// The directions of node (x, y) that a boundary-free body (SKIP) does not store:
+// all nine of a node that the boundary-node pass of the same launch recomputes
+// (0x1FF); under a pressure rewrite done by that pass, the rewritten ones of
+// columns 0 and nx-1.  Evaluated where the node is stored, in chunks that may
+// hold such nodes only: nothing of it stays in registers across the body, which
+// runs at its register cap.
+template <bool EDGES, bool PASS_PRESSURE>
+__device__ __forceinline__ uint32_t pass_skip(const GeoK& g, int x, int y) {
+  uint32_t d = frame_desc(g, x, y);
+  if (d == 0u && g.bcmask != nullptr && x >= g.box_x0 && x <= g.box_x1 && y >= g.box_y0 && y <= g.box_y1 &&
+      ((__ldg(g.bcmask + y * g.words + (x >> 5)) >> (x & 31)) & 1u))
+    d = __ldg(g.desc + y * g.nx + x);
+  if (EDGES && ((x == 0 && d == g.edge_in_desc) || (x == g.nx - 1 && d == g.edge_out_desc))) d = 0u;
+  if (PASS_PRESSURE && g.pressure && (x == 1 || x == g.nx - 2)) return 0x1FFu;
+  if ((d & 0x3FFFFu) != 0u) return 0x1FFu;
+  if (PASS_PRESSURE && g.pressure) return x == 0 ? g.pin : (x == g.nx - 1 ? g.pout : 0u);
+  return 0u;
 }
 
 // ---- one node's (or pair's) collision, shared by every fused body ---------------
@@ -210,10 +261,11 @@ __device__ __forceinline__ void collide_pair(float2 g2[9], float2& sum, float2& 
 // 32-bit element indices (9 * plane < 2^31).  Boundary descriptors and the
 // pressure rewrite are compiled in only where a geometry may have them.
 // ---------------------------------------------------------------------------
-template <int STORE, int NPT, bool HAS_BC, bool HAS_PRESSURE, bool EDGES = false, bool SHIFT = false>
+template <int STORE, int NPT, bool HAS_BC, bool HAS_PRESSURE, bool EDGES = false, bool SHIFT = false,
+          bool SKIP = false, bool INSIDE = false>
 __device__ __forceinline__ void fused_v2_body(const KParams& P, const void* pop_in_v, void* pop_out_v,
                                               const void* aux_in_v, void* aux_out_v, int x0, int y,
-                                              uint32_t seed, bool listed = false) {
+                                              uint32_t seed, bool listed = false, bool special = true) {
   using St = Store<STORE>;
   using T = typename St::T;
   using R = typename St::R;
@@ -228,16 +280,16 @@ __device__ __forceinline__ void fused_v2_body(const KParams& P, const void* pop_
   const int lane = threadIdx.x & 31;
   const int nx = P.g.nx, ny = P.g.ny;
   const int xlast = ((nx - 1) / NPT) * NPT;  // first node of the last chunk of a row
-  const bool active = x0 < nx;
+  const bool active = INSIDE || x0 < nx;
   if (!active) x0 = xlast;  // stays in the shuffles, stores nothing
-  const int nvalid = min(NPT, nx - x0);
+  const int nvalid = INSIDE ? NPT : min(NPT, nx - x0);
   const int pitch = (int)P.pitch, plane = (int)P.plane;
-  const int ym = y == 0 ? ny - 1 : y - 1, yp = y == ny - 1 ? 0 : y + 1;
+  const int ym = !INSIDE && y == 0 ? ny - 1 : y - 1, yp = !INSIDE && y == ny - 1 ? 0 : y + 1;
   const int r0 = y * pitch, rm = ym * pitch, rp = yp * pitch;
-  const bool first = x0 == 0;
-  const bool last = x0 == xlast;
+  const bool first = !INSIDE && x0 == 0;
+  const bool last = !INSIDE && x0 == xlast;
   const int xm = first ? nx - 1 : x0 - 1;
-  const int xp = x0 + NPT >= nx ? 0 : x0 + NPT;
+  const int xp = !INSIDE && x0 + NPT >= nx ? 0 : x0 + NPT;
   const T* pin = static_cast<const T*>(pop_in_v);
   auto ld_work = [&](const T* p, int i) -> R {
     if constexpr (SH) return St::ld_dev(p);
@@ -367,7 +419,12 @@ __device__ __forceinline__ void fused_v2_body(const KParams& P, const void* pop_
     }
   }
 
-  if (aux_out_v != nullptr && active && x0 <= nx - 2 && nx - 2 < x0 + NPT) {
+  // the directions of a node that the boundary-node pass stores instead
+  auto skipped = [&](int x) -> uint32_t {
+    if constexpr (SKIP) return pass_skip<EDGES, !HAS_PRESSURE>(P.g, x, y);
+    else return 0u;
+  };
+  if (!INSIDE && aux_out_v != nullptr && active && x0 <= nx - 2 && nx - 2 < x0 + NPT) {
     // the outlet memory holds full populations in every kernel
     R* aux_out = static_cast<R*>(aux_out_v);
     const int ka = nx - 2 - x0;
@@ -378,9 +435,11 @@ __device__ __forceinline__ void fused_v2_body(const KParams& P, const void* pop_
       a6 = k == ka ? f[6][k] : a6;
       a7 = k == ka ? f[7][k] : a7;
     }
-    aux_out[0 * ny + y] = f_of_work(a3, 3);
-    aux_out[1 * ny + y] = f_of_work(a6, 6);
-    aux_out[2 * ny + y] = f_of_work(a7, 7);
+    if (skipped(nx - 2) != 0x1FFu) {
+      aux_out[0 * ny + y] = f_of_work(a3, 3);
+      aux_out[1 * ny + y] = f_of_work(a6, 6);
+      aux_out[2 * ny + y] = f_of_work(a7, 7);
+    }
   }
 
   R pv[9];  // pressure rewrite computed by the node at column nx-2 or 1
@@ -392,15 +451,15 @@ __device__ __forceinline__ void fused_v2_body(const KParams& P, const void* pop_
   auto node_extras = [&](int k, R sum, R rho, R ux, R uy, const R g[9]) {
     const int x = x0 + k;
     if (want_m && active && k < nvalid) {
-      if (P.rho_out.p != nullptr) {
+      if (P.rho_out.p != nullptr && skipped(x) != 0x1FFu) {
         P.rho_out.p[x * P.rho_out.sx + y * P.rho_out.sy] = SH ? 1.0 + (double)sum / (double)kS : (double)rho;
         double* up = P.u_out.p + x * P.u_out.sx + y * P.u_out.sy;
         up[0] = (double)ux;
         up[P.u_out.sc] = (double)uy;
       }
-      write_probe(P, x, y, ux, uy, !HAS_BC, EDGES);
+      write_probe(P, x, y, ux, uy, !HAS_BC, EDGES, !HAS_PRESSURE);
     }
-    if (HAS_PRESSURE && P.g.pressure && k < nvalid && (x == nx - 2 || x == 1)) {
+    if (HAS_PRESSURE && P.g.pressure && k < nvalid && (x == nx - 2 || x == 1) && skipped(x) != 0x1FFu) {
       R br[9];
       bracket9_fast(ux, uy, br);
       const R rb = (R)(x == nx - 2 ? P.g.rho_in : P.g.rho_out) * kS - rho;
@@ -462,7 +521,7 @@ __device__ __forceinline__ void fused_v2_body(const KParams& P, const void* pop_
   for (int k = 0; k < NPT; ++k) hk[k] = sr ? mix32((uint32_t)(y * nx + x0 + k) * 0x9E3779B1u ^ seed) : 0u;
   T* pout = static_cast<T*>(pop_out_v);
   const bool pr = HAS_PRESSURE && P.g.pressure;
-  if (nvalid == NPT && !(pr && (first || last))) {
+  if (nvalid == NPT && !(pr && (first || last)) && (!SKIP || !special)) {
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
       T raw[NPT];
@@ -474,16 +533,22 @@ __device__ __forceinline__ void fused_v2_body(const KParams& P, const void* pop_
       st_vec<T, NPT>(pout + i * plane + r0 + x0, raw);
     }
   } else {
-    // partial chunk, or a row end under the pressure rewrite: column 0 skips the
-    // inlet-side directions, column nx-1 the outlet side
+    // partial chunk, a chunk with nodes of the pass, or a row end under the
+    // pressure rewrite: column 0 skips the inlet-side directions, column nx-1 the
+    // outlet side
+    uint32_t skip[SKIP ? NPT : 1] = {};
+    if constexpr (SKIP) {
+#pragma unroll
+      for (int k = 0; k < NPT; ++k) skip[k] = k < nvalid ? skipped(x0 + k) : 0u;
+    }
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
 #pragma unroll
       for (int k = 0; k < NPT; ++k) {
         const int x = x0 + k;
-        const bool skip = k >= nvalid || (pr && ((x == 0 && ((P.g.pin >> i) & 1u)) ||
-                                                 (x == nx - 1 && ((P.g.pout >> i) & 1u))));
-        if (!skip) pout[i * plane + r0 + x] = to_store(f[i][k], i, hk[k]);
+        const bool drop = k >= nvalid || (SKIP && ((skip[SKIP ? k : 0] >> i) & 1u)) ||
+                          (pr && ((x == 0 && ((P.g.pin >> i) & 1u)) || (x == nx - 1 && ((P.g.pout >> i) & 1u))));
+        if (!drop) pout[i * plane + r0 + x] = to_store(f[i][k], i, hk[k]);
         hk[k] = hk[k] * 0x2C1B3C6Du + 0x297A2D39u;
       }
     }
@@ -509,9 +574,10 @@ __device__ __forceinline__ void fused_v2_body(const KParams& P, const void* pop_
 // use float64 on the converted values.
 // The outlet memory holds the stored integers, as in the generic kernel.
 // ---------------------------------------------------------------------------
-template <int NPT, bool HAS_BC, bool HAS_PRESSURE, bool EDGES = false>
+template <int NPT, bool HAS_BC, bool HAS_PRESSURE, bool EDGES = false, bool SKIP = false>
 __device__ __forceinline__ void fused_fx_body(const KParams& P, const void* pop_in_v, void* pop_out_v,
-                                              const void* aux_in_v, void* aux_out_v, int x0, int y) {
+                                              const void* aux_in_v, void* aux_out_v, int x0, int y,
+                                              bool special = true) {
   using T = long long;
   const int lane = threadIdx.x & 31;
   const int nx = P.g.nx, ny = P.g.ny;
@@ -530,6 +596,9 @@ __device__ __forceinline__ void fused_fx_body(const KParams& P, const void* pop_
 
   // the boundary mask word first: its latency overlaps the population loads
   const bool has_bc = HAS_BC && P.g.bcmask != nullptr;
+  // the boundary constants come as fixed-point numbers (set_fx_tables)
+  auto kconst = [&](int set, int i) { return __double_as_longlong(P.g.kconst[set][i]); };
+  auto cconst = [&](int set, int i) { return __double_as_longlong(P.g.cconst[set][i]); };
   const uint32_t bcword = has_bc ? __ldg(P.g.bcmask + y * P.g.words + (x0 >> 5)) : 0u;
   T f[9][NPT];
 #pragma unroll
@@ -575,7 +644,7 @@ __device__ __forceinline__ void fused_fx_body(const KParams& P, const void* pop_
     // nx-1 (the pass recomputes the ones with other sources)
     if (first && P.g.edge_in_desc != 0u) {
 #pragma unroll
-      for (int i = 0; i < 9; ++i) f[i][0] = fx::to_fx(P.g.edge_in_f[i], wd(i));
+      for (int i = 0; i < 9; ++i) f[i][0] = __double_as_longlong(P.g.edge_in_f[i]);
     }
     if (last && P.g.edge_out_desc != 0u && aux_in_v != nullptr) {
       const T* aux_in = static_cast<const T*>(aux_in_v);
@@ -604,9 +673,9 @@ __device__ __forceinline__ void fused_fx_body(const KParams& P, const void* pop_
         for (int i = 0; i < 9; ++i) {
           const uint32_t s = (d >> (2 * i)) & 3u;
           if (s == LBM_SRC_BOUNCE)
-            f[i][k] = pin[opp(i) * plane + r0 + x] - fx::round_scaled(P.g.kconst[ks][i], fx::kS);
+            f[i][k] = pin[opp(i) * plane + r0 + x] - kconst(ks, i);
           else if (s == LBM_SRC_CONST)
-            f[i][k] = fx::to_fx(P.g.cconst[cs][i], wd(i));
+            f[i][k] = cconst(cs, i);
           else if (s == LBM_SRC_OUTLET && outlet_slot(i) >= 0 && aux_in != nullptr)
             f[i][k] = aux_in[outlet_slot(i) * ny + y];
         }
@@ -614,6 +683,11 @@ __device__ __forceinline__ void fused_fx_body(const KParams& P, const void* pop_
     }
   }
 
+  // the directions of a node that the boundary-node pass stores instead
+  auto skipped = [&](int x) -> uint32_t {
+    if constexpr (SKIP) return pass_skip<EDGES, !HAS_PRESSURE>(P.g, x, y);
+    else return 0u;
+  };
   if (aux_out_v != nullptr && active && x0 <= nx - 2 && nx - 2 < x0 + NPT) {
     T* aux_out = static_cast<T*>(aux_out_v);
     const int ka = nx - 2 - x0;
@@ -624,9 +698,11 @@ __device__ __forceinline__ void fused_fx_body(const KParams& P, const void* pop_
       a6 = k == ka ? f[6][k] : a6;
       a7 = k == ka ? f[7][k] : a7;
     }
-    aux_out[0 * ny + y] = a3;
-    aux_out[1 * ny + y] = a6;
-    aux_out[2 * ny + y] = a7;
+    if (skipped(nx - 2) != 0x1FFu) {
+      aux_out[0 * ny + y] = a3;
+      aux_out[1 * ny + y] = a6;
+      aux_out[2 * ny + y] = a7;
+    }
   }
 
   T pv[9];  // pressure rewrite computed by the node at column nx-2 or 1
@@ -638,7 +714,7 @@ __device__ __forceinline__ void fused_fx_body(const KParams& P, const void* pop_
 #pragma unroll
     for (int i = 0; i < 9; ++i) g[i] = f[i][k];
     const int x = x0 + k;
-    const bool pnode = HAS_PRESSURE && P.g.pressure && k < nvalid && (x == nx - 2 || x == 1);
+    const bool pnode = HAS_PRESSURE && P.g.pressure && k < nvalid && (x == nx - 2 || x == 1) && skipped(x) != 0x1FFu;
     const bool out = want_m && active && k < nvalid &&
                      (P.rho_out.p != nullptr || (P.probe_buf != nullptr && x == P.probe_x && y == P.probe_y));
     if (out) {
@@ -648,13 +724,13 @@ __device__ __forceinline__ void fused_fx_body(const KParams& P, const void* pop_
       const double rho = density9(d);
       double ux, uy;
       velocity_fast(d, rho, ux, uy);
-      if (P.rho_out.p != nullptr) {
+      if (P.rho_out.p != nullptr && skipped(x) != 0x1FFu) {
         P.rho_out.p[x * P.rho_out.sx + y * P.rho_out.sy] = rho;
         double* up = P.u_out.p + x * P.u_out.sx + y * P.u_out.sy;
         up[0] = ux;
         up[P.u_out.sc] = uy;
       }
-      write_probe(P, x, y, ux, uy, !HAS_BC, EDGES);
+      write_probe(P, x, y, ux, uy, !HAS_BC, EDGES, !HAS_PRESSURE);
     }
     if (pnode) {
       int64_t q[9];
@@ -672,18 +748,23 @@ __device__ __forceinline__ void fused_fx_body(const KParams& P, const void* pop_
   if (!active) return;
   T* pout = static_cast<T*>(pop_out_v);
   const bool pr = HAS_PRESSURE && P.g.pressure;
-  if ((NPT == 1 || nvalid == NPT) && !(pr && (first || last))) {
+  if ((NPT == 1 || nvalid == NPT) && !(pr && (first || last)) && (!SKIP || !special)) {
 #pragma unroll
     for (int i = 0; i < 9; ++i) st_vec<T, NPT>(pout + i * plane + r0 + x0, f[i]);
   } else {
+    uint32_t skip[SKIP ? NPT : 1] = {};
+    if constexpr (SKIP) {
+#pragma unroll
+      for (int k = 0; k < NPT; ++k) skip[k] = k < nvalid ? skipped(x0 + k) : 0u;
+    }
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
 #pragma unroll
       for (int k = 0; k < NPT; ++k) {
         const int x = x0 + k;
-        const bool skip = k >= nvalid || (pr && ((x == 0 && ((P.g.pin >> i) & 1u)) ||
-                                                 (x == nx - 1 && ((P.g.pout >> i) & 1u))));
-        if (!skip) pout[i * plane + r0 + x] = f[i][k];
+        const bool drop = k >= nvalid || (SKIP && ((skip[SKIP ? k : 0] >> i) & 1u)) ||
+                          (pr && ((x == 0 && ((P.g.pin >> i) & 1u)) || (x == nx - 1 && ((P.g.pout >> i) & 1u))));
+        if (!drop) pout[i * plane + r0 + x] = f[i][k];
       }
     }
   }
@@ -788,6 +869,12 @@ inline bool to_geok(const lbm_geometry* g, GeoK& k) {
     return set_error(LBM_ERR_ARG, "the deviation reference velocity must lie inside (-0.5, 0.5)"), false;
   k.dev_ref_ux = ux;
   k.dev_ref_uy = uy;
+  const bool framed = g->frame != 0 && g->nx >= 3 && g->ny >= 3;
+  if (framed) std::memcpy(k.frame_desc, g->frame_desc, sizeof(k.frame_desc));
+  k.box_x0 = framed ? g->inner_box[0] : 0;
+  k.box_x1 = framed ? g->inner_box[1] : g->nx - 1;
+  k.box_y0 = framed ? g->inner_box[2] : 0;
+  k.box_y1 = framed ? g->inner_box[3] : g->ny - 1;
   return true;
 }
 
@@ -832,6 +919,20 @@ inline void set_shift(KParams& P) {
     h.sx = (float)mx;
     h.sy = (float)my;
   }
+}
+
+// The fixed-point step bodies read their boundary constants as fixed-point
+// numbers: replaces the float64 tables by the bits of the numbers the bodies
+// would round them to at every boundary node.
+inline void set_fx_tables(GeoK& g) {
+  auto put = [](double& slot, int64_t q) { std::memcpy(&slot, &q, 8); };
+  for (int s = 0; s < LBM_MAX_SETS; ++s) {
+    for (int i = 0; i < 9; ++i) {
+      put(g.kconst[s][i], fx::round_scaled(g.kconst[s][i], fx::kS));
+      put(g.cconst[s][i], fx::to_fx(g.cconst[s][i], wd(i)));
+    }
+  }
+  for (int i = 0; i < 9; ++i) put(g.edge_in_f[i], fx::to_fx(g.edge_in_f[i], wd(i)));
 }
 
 inline int check_omega(double omega) {

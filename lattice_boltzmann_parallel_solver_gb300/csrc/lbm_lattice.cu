@@ -191,36 +191,19 @@ __global__ void __launch_bounds__(256) lattice_kernel(const __grid_constant__ KP
   }
 }
 
-// the float32 and 16-bit storages: registers capped so that 1024 threads fit
-// on an SM; SHIFT: the reference-shifted 16-bit storages
-template <int STORE, int NPT, int THREADS, bool SHIFT, bool HAS_BC, bool HAS_PRESSURE>
-__global__ void __launch_bounds__(THREADS, (STORE == LBM_STORE_F16S || STORE == LBM_STORE_BF16S ||
-                                            (STORE == LBM_STORE_F32 && NPT <= 2))
-                                               ? 1024 / THREADS
-                                               : 1)
-    fused_v2_kernel(const __grid_constant__ KParams P) {
-  pdl_wait();
-  fused_v2_body<STORE, NPT, HAS_BC, HAS_PRESSURE, false, SHIFT>(P, P.pop_in, P.pop_out, P.aux_in, P.aux_out,
-                                                                (blockIdx.x * THREADS + threadIdx.x) * NPT,
-                                                                blockIdx.y, launch_seed(P));
-}
+// How a vectorised step's kernel applies the boundary sources: kBcNone without
+// any, kBcInline inside the body, kBcPass (float32) in the first pass_rows rows of
+// blocks, one thread per listed boundary node, beside the blocks of a body that
+// leaves those nodes out.
+enum { kBcNone = 0, kBcInline = 1, kBcPass = 2 };
 
-// one node per thread: registers capped so that 1024 threads fit on an SM
-template <int NPT, int THREADS, bool HAS_BC, bool HAS_PRESSURE>
-__global__ void __launch_bounds__(THREADS, NPT == 1 ? 1024 / THREADS : 1) fused_fx_kernel(const __grid_constant__ KParams P) {
-  pdl_wait();
-  fused_fx_body<NPT, HAS_BC, HAS_PRESSURE>(P, P.pop_in, P.pop_out, P.aux_in, P.aux_out,
-                                           (blockIdx.x * THREADS + threadIdx.x) * NPT, blockIdx.y);
-}
-
-// The boundary-node pass: after a vectorised step ran its boundary-free body
-// over every node, one thread per listed boundary node recomputes that node
-// with its sources (the same body at one node per thread, so the arithmetic and
-// the random bits are those of the in-step path) and overwrites its outputs.
+// The boundary-node pass, one thread per listed boundary node: recomputes the
+// node with its sources (the same body at one node per thread, so the arithmetic
+// and the random bits are those of the sources inside the step).  It is bound by
+// the latency of its dependent loads.
 template <int STORE, int THREADS, bool HAS_PRESSURE, bool SHIFT>
-__global__ void __launch_bounds__(THREADS) fixup_v2_kernel(const __grid_constant__ KParams P) {
-  pdl_wait();
-  const int t = blockIdx.x * THREADS + threadIdx.x;
+__device__ __forceinline__ void pass_block(const KParams& P) {
+  const int t = (int)((blockIdx.y * gridDim.x + blockIdx.x) * THREADS + threadIdx.x);
   if (t >= P.g.n_bcnodes) return;
   const int node = __ldg(P.g.bcnodes + t);
   const int y = node / P.g.nx, x = node - y * P.g.nx;
@@ -229,6 +212,57 @@ __global__ void __launch_bounds__(THREADS) fixup_v2_kernel(const __grid_constant
   else
     fused_v2_body<STORE, 1, true, HAS_PRESSURE, false, SHIFT>(P, P.pop_in, P.pop_out, P.aux_in, P.aux_out, x, y,
                                                               launch_seed(P), true);
+}
+
+// The pass as a launch of its own, after a boundary-free step over every node:
+// it overwrites the listed nodes' outputs.
+template <int STORE, int THREADS, bool HAS_PRESSURE, bool SHIFT>
+__global__ void __launch_bounds__(THREADS) fixup_v2_kernel(const __grid_constant__ KParams P) {
+  pdl_wait();
+  pass_block<STORE, THREADS, HAS_PRESSURE, SHIFT>(P);
+}
+
+// the float32 and 16-bit storages: registers capped so that 1024 threads fit on
+// an SM (float32 at 4 nodes per thread: 640); SHIFT: the reference-shifted
+// 16-bit storages.  In float32 a warp whose nodes are all inside (see inside())
+// takes a body without wrap, outlet memory and pressure code (4096^2: 194 ->
+// 174 us); in the others, nearer to their register cap, a second body costs more
+// than it saves.
+template <int STORE, int NPT, int THREADS, bool SHIFT, int BC, bool HAS_PRESSURE>
+__global__ void __launch_bounds__(THREADS, (STORE == LBM_STORE_F16S || STORE == LBM_STORE_BF16S ||
+                                            (STORE == LBM_STORE_F32 && NPT <= 2))
+                                               ? 1024 / THREADS
+                                               : (STORE == LBM_STORE_F32 ? 640 / THREADS : 1))
+    fused_v2_kernel(const __grid_constant__ KParams P) {
+  pdl_wait();
+  int y = (int)blockIdx.y;
+  if constexpr (BC == kBcPass) {
+    if (y < P.pass_rows) {
+      pass_block<STORE, THREADS, HAS_PRESSURE, SHIFT>(P);
+      return;
+    }
+    y -= P.pass_rows;
+  }
+  const int t = (int)(blockIdx.x * THREADS + threadIdx.x);
+  if constexpr (STORE == LBM_STORE_F32 && BC != kBcInline) {
+    const int xa = (t & ~31) * NPT;
+    if (inside(P.g, BC == kBcPass, xa, xa + 32 * NPT - 1, y)) {
+      fused_v2_body<STORE, NPT, false, false, false, SHIFT, false, true>(P, P.pop_in, P.pop_out, P.aux_in, P.aux_out,
+                                                                         t * NPT, y, launch_seed(P));
+      return;
+    }
+  }
+  fused_v2_body<STORE, NPT, BC == kBcInline, HAS_PRESSURE, false, SHIFT, BC == kBcPass>(
+      P, P.pop_in, P.pop_out, P.aux_in, P.aux_out, t * NPT, y, launch_seed(P), false,
+      BC == kBcPass && pass_chunk(P.g, (int)blockIdx.x * (THREADS * NPT), THREADS * NPT, y));
+}
+
+// one node per thread: registers capped so that 1024 threads fit on an SM
+template <int NPT, int THREADS, int BC, bool HAS_PRESSURE>
+__global__ void __launch_bounds__(THREADS, NPT == 1 ? 1024 / THREADS : 1) fused_fx_kernel(const __grid_constant__ KParams P) {
+  pdl_wait();
+  fused_fx_body<NPT, BC == kBcInline, HAS_PRESSURE>(P, P.pop_in, P.pop_out, P.aux_in, P.aux_out,
+                                                    (blockIdx.x * THREADS + threadIdx.x) * NPT, blockIdx.y);
 }
 
 // adds the steps of a lbm_lattice_run_opts call to its device step counter
@@ -277,38 +311,45 @@ static int dispatch(int storage, bool exact, const KParams& P, cudaStream_t s) {
 
 constexpr int kV2Threads = 128;
 
-// the four boundary specialisations of one vectorised kernel
-#define LBM_LAUNCH_SPECIALISED(KERNEL, ...)                                            \
-  do {                                                                                 \
-    const bool bc = P.g.bcmask != nullptr, pr = P.g.pressure != 0;                     \
-    if (bc && pr)                                                                      \
-      launch_step(KERNEL<__VA_ARGS__, true, true>, grid, kV2Threads, overlap, s, 0, P);   \
-    else if (bc)                                                                       \
-      launch_step(KERNEL<__VA_ARGS__, true, false>, grid, kV2Threads, overlap, s, 0, P);  \
-    else if (pr)                                                                       \
-      launch_step(KERNEL<__VA_ARGS__, false, true>, grid, kV2Threads, overlap, s, 0, P);  \
-    else                                                                               \
-      launch_step(KERNEL<__VA_ARGS__, false, false>, grid, kV2Threads, overlap, s, 0, P); \
+// the boundary specialisations of one vectorised kernel; PASS: with kBcPass
+#define LBM_LAUNCH_SPECIALISED(PASS, KERNEL, ...)                                                       \
+  do {                                                                                                  \
+    const bool pr = P.g.pressure != 0;                                                                  \
+    if constexpr (PASS) {                                                                               \
+      if (bc == kBcPass && pr)                                                                          \
+        launch_step(KERNEL<__VA_ARGS__, kBcPass, true>, grid, kV2Threads, overlap, s, 0, P);            \
+      else if (bc == kBcPass)                                                                           \
+        launch_step(KERNEL<__VA_ARGS__, kBcPass, false>, grid, kV2Threads, overlap, s, 0, P);           \
+    }                                                                                                   \
+    if (bc == kBcInline && pr)                                                                          \
+      launch_step(KERNEL<__VA_ARGS__, kBcInline, true>, grid, kV2Threads, overlap, s, 0, P);            \
+    else if (bc == kBcInline)                                                                           \
+      launch_step(KERNEL<__VA_ARGS__, kBcInline, false>, grid, kV2Threads, overlap, s, 0, P);           \
+    else if (bc == kBcNone && pr)                                                                       \
+      launch_step(KERNEL<__VA_ARGS__, kBcNone, true>, grid, kV2Threads, overlap, s, 0, P);              \
+    else if (bc == kBcNone)                                                                             \
+      launch_step(KERNEL<__VA_ARGS__, kBcNone, false>, grid, kV2Threads, overlap, s, 0, P);             \
   } while (0)
 
 template <int NPT>
-static dim3 v2_grid(const KParams& P) {
-  const int chunks = (P.g.nx + NPT - 1) / NPT;
-  return dim3((unsigned)((chunks + kV2Threads - 1) / kV2Threads), (unsigned)P.g.ny, 1);
+static int v2_blocks(const KParams& P) {
+  return ((P.g.nx + NPT - 1) / NPT + kV2Threads - 1) / kV2Threads;
 }
 
 template <int STORE, int NPT, bool SHIFT = false>
-static int launch_v2(const KParams& P, bool overlap, cudaStream_t s) {
-  const dim3 grid = v2_grid<NPT>(P);
-  LBM_LAUNCH_SPECIALISED(fused_v2_kernel, STORE, NPT, kV2Threads, SHIFT);
+static int launch_v2(KParams P, int bc, bool overlap, cudaStream_t s) {
+  const int bx = v2_blocks<NPT>(P);
+  P.pass_rows = bc == kBcPass ? (P.g.n_bcnodes + kV2Threads * bx - 1) / (kV2Threads * bx) : 0;
+  const dim3 grid((unsigned)bx, (unsigned)(P.g.ny + P.pass_rows));
+  LBM_LAUNCH_SPECIALISED(STORE == LBM_STORE_F32, fused_v2_kernel, STORE, NPT, kV2Threads, SHIFT);
   count_launch();
   return check_launch("fused_v2_kernel");
 }
 
 template <int NPT>
-static int launch_fx(const KParams& P, bool overlap, cudaStream_t s) {
-  const dim3 grid = v2_grid<NPT>(P);
-  LBM_LAUNCH_SPECIALISED(fused_fx_kernel, NPT, kV2Threads);
+static int launch_fx(const KParams& P, int bc, bool overlap, cudaStream_t s) {
+  const dim3 grid((unsigned)v2_blocks<NPT>(P), (unsigned)P.g.ny);
+  LBM_LAUNCH_SPECIALISED(false, fused_fx_kernel, NPT, kV2Threads);
   count_launch();
   return check_launch("fused_fx_kernel");
 }
@@ -346,8 +387,8 @@ static bool tile_applies(int storage, int flags, const KParams& P) {
 
 constexpr int kFixupThreads = 128;
 
-template <int STORE, bool SHIFT = false>
 // (always right after the step kernel of the same launch_fused)
+template <int STORE, bool SHIFT = false>
 static int launch_fixup(const KParams& P, cudaStream_t s) {
   const dim3 grid((unsigned)((P.g.n_bcnodes + kFixupThreads - 1) / kFixupThreads));
   if (P.g.pressure)
@@ -358,64 +399,64 @@ static int launch_fixup(const KParams& P, cudaStream_t s) {
   return check_launch("fixup_v2_kernel");
 }
 
-static int launch_fused_step(int storage, int npt, int flags, const KParams& P, bool overlap, cudaStream_t s);
-
-// One step.  On large lattices whose geometry lists its boundary nodes (at most
-// an eighth of the lattice), the vectorised kernel runs without boundary work:
-// the body's boundary block then stays out of the hot loop (it costs registers
-// under the 64-register cap), and the listed nodes are recomputed by the
-// boundary-node pass.  Smaller lattices keep one launch per step, whose fixed
-// cost would otherwise outweigh the gain.  Measured on the cavity (split against
-// inline GLUPS): the 16-bit storages gain from 2896^2 on (132 against 124) and
-// lose below 2048^2 (64 against 85 at 1024^2); the other storages gain only at
-// 8192^2 (fx64 46.9 against 46.5) and lose or tie up to 4096^2.
-static int64_t split_nodes(int storage) {
-  return (storage == LBM_STORE_F16S || storage == LBM_STORE_BF16S || ref_shifted(storage)) ? (int64_t)1 << 22
-                                                                                              : (int64_t)1 << 25;
+static int launch_fused_step(int storage, int npt, int bc, int flags, const KParams& P, bool overlap, cudaStream_t s) {
+  switch (storage * 16 + npt) {
+    case LBM_STORE_F64 * 16 + 2: return launch_v2<LBM_STORE_F64, 2>(P, bc, overlap, s);
+    case LBM_STORE_F64 * 16 + 4: return launch_v2<LBM_STORE_F64, 4>(P, bc, overlap, s);
+    case LBM_STORE_FX64 * 16 + 1: return launch_fx<1>(P, bc, overlap, s);
+    case LBM_STORE_FX64 * 16 + 2: return launch_fx<2>(P, bc, overlap, s);
+    case LBM_STORE_FX64 * 16 + 4: return launch_fx<4>(P, bc, overlap, s);
+    case LBM_STORE_F32 * 16 + 2: return launch_v2<LBM_STORE_F32, 2>(P, bc, overlap, s);
+    case LBM_STORE_F32 * 16 + 4: return launch_v2<LBM_STORE_F32, 4>(P, bc, overlap, s);
+    case LBM_STORE_F16S * 16 + 2: return launch_v2<LBM_STORE_F16S, 2>(P, bc, overlap, s);
+    case LBM_STORE_F16S * 16 + 4: return launch_v2<LBM_STORE_F16S, 4>(P, bc, overlap, s);
+    case LBM_STORE_F16S * 16 + 8: return launch_v2<LBM_STORE_F16S, 8>(P, bc, overlap, s);
+    case LBM_STORE_BF16S * 16 + 2: return launch_v2<LBM_STORE_BF16S, 2>(P, bc, overlap, s);
+    case LBM_STORE_BF16S * 16 + 4: return launch_v2<LBM_STORE_BF16S, 4>(P, bc, overlap, s);
+    case LBM_STORE_BF16S * 16 + 8: return launch_v2<LBM_STORE_BF16S, 8>(P, bc, overlap, s);
+    case LBM_STORE_F16R * 16 + 4: return launch_v2<LBM_STORE_F16S, 4, true>(P, bc, overlap, s);
+    case LBM_STORE_BF16R * 16 + 4: return launch_v2<LBM_STORE_BF16S, 4, true>(P, bc, overlap, s);
+    default: return dispatch<MODE_FUSED>(storage, flags & LBM_FLAG_EXACT, P, s);
+  }
 }
 
+// One step.  A geometry that lists its boundary nodes (at most an eighth of the
+// lattice) may leave them to the boundary-node pass; a probe keeps the sources
+// inside the step, so its node is recorded once.
+//
+// float32 takes the pass in blocks of the step's own launch, at every size: its
+// body is far from its register cap, and with the sources inside, the warps at a
+// row's ends wait for mask, descriptor and bounced populations in turn.  Cavity,
+// us per step, inside against pass: 1024^2 12.5 / 10.7, 2048^2 55.3 / 47.5, 4096^2
+// 195 / 178, 8192^2 759 / 698.  In the other storages leaving the nodes out costs
+// the capped body more than the pass saves (4096^2 f16 117 against 107, fx64 377
+// against 367), so they keep the sources inside, and from 2^25 nodes take the pass
+// as a second launch (8192^2 fx64 1437 against 1444).
 static int launch_fused(int storage, int flags, const KParams& P, bool overlap, cudaStream_t s) {
   const int npt = v2_npt(storage, flags, P);
   const int64_t nodes = (int64_t)P.g.nx * P.g.ny;
-  // a probe keeps the sources inside the step, so its node is recorded once
-  const bool split = npt > 0 && !(flags & LBM_FLAG_BC_INLINE) && P.g.bcmask != nullptr && P.g.n_bcnodes > 0 &&
-                     P.probe_buf == nullptr &&
-                     (nodes >= split_nodes(storage) || (flags & LBM_FLAG_BC_SPLIT)) &&
-                     (int64_t)P.g.n_bcnodes * 8 <= nodes;
-  if (!split) return launch_fused_step(storage, npt, flags, P, overlap, s);
+  const bool listed = npt > 0 && !(flags & LBM_FLAG_BC_INLINE) && P.g.bcmask != nullptr && P.g.n_bcnodes > 0 &&
+                      P.probe_buf == nullptr && (int64_t)P.g.n_bcnodes * 8 <= nodes;
+  const int inside = P.g.bcmask != nullptr ? kBcInline : kBcNone;
+  if (!listed) return launch_fused_step(storage, npt, inside, flags, P, overlap, s);
+  if (storage == LBM_STORE_F32) {
+    // the pass's rows of blocks fit the grid beside the lattice's
+    const bool fits = (int64_t)P.g.ny + P.g.n_bcnodes / kV2Threads + 1 <= 65535;
+    return launch_fused_step(storage, npt, fits ? kBcPass : inside, flags, P, overlap, s);
+  }
+  if (nodes < ((int64_t)1 << 25) && !(flags & LBM_FLAG_BC_SPLIT))
+    return launch_fused_step(storage, npt, inside, flags, P, overlap, s);
   KParams Q = P;
   Q.g.bcmask = nullptr;
-  if (int e = launch_fused_step(storage, npt, flags, Q, overlap, s)) return e;
+  if (int e = launch_fused_step(storage, npt, kBcNone, flags, Q, overlap, s)) return e;
   switch (storage) {
     case LBM_STORE_F64: return launch_fixup<LBM_STORE_F64>(P, s);
-    case LBM_STORE_F32: return launch_fixup<LBM_STORE_F32>(P, s);
     case LBM_STORE_F16S: return launch_fixup<LBM_STORE_F16S>(P, s);
     case LBM_STORE_BF16S: return launch_fixup<LBM_STORE_BF16S>(P, s);
     case LBM_STORE_FX64: return launch_fixup<LBM_STORE_FX64>(P, s);
     case LBM_STORE_F16R: return launch_fixup<LBM_STORE_F16S, true>(P, s);
     case LBM_STORE_BF16R: return launch_fixup<LBM_STORE_BF16S, true>(P, s);
     default: return set_error(LBM_ERR_ARG, "unknown storage type");
-  }
-}
-
-static int launch_fused_step(int storage, int npt, int flags, const KParams& P, bool overlap, cudaStream_t s) {
-  switch (storage * 16 + npt) {
-    case LBM_STORE_F64 * 16 + 2: return launch_v2<LBM_STORE_F64, 2>(P, overlap, s);
-    case LBM_STORE_F64 * 16 + 4: return launch_v2<LBM_STORE_F64, 4>(P, overlap, s);
-    case LBM_STORE_FX64 * 16 + 1: return launch_fx<1>(P, overlap, s);
-    case LBM_STORE_FX64 * 16 + 2: return launch_fx<2>(P, overlap, s);
-    case LBM_STORE_FX64 * 16 + 4: return launch_fx<4>(P, overlap, s);
-    case LBM_STORE_F32 * 16 + 2: return launch_v2<LBM_STORE_F32, 2>(P, overlap, s);
-    case LBM_STORE_F32 * 16 + 4: return launch_v2<LBM_STORE_F32, 4>(P, overlap, s);
-    case LBM_STORE_F16S * 16 + 2: return launch_v2<LBM_STORE_F16S, 2>(P, overlap, s);
-    case LBM_STORE_F16S * 16 + 4: return launch_v2<LBM_STORE_F16S, 4>(P, overlap, s);
-    case LBM_STORE_F16S * 16 + 8: return launch_v2<LBM_STORE_F16S, 8>(P, overlap, s);
-    case LBM_STORE_BF16S * 16 + 2: return launch_v2<LBM_STORE_BF16S, 2>(P, overlap, s);
-    case LBM_STORE_BF16S * 16 + 4: return launch_v2<LBM_STORE_BF16S, 4>(P, overlap, s);
-    case LBM_STORE_BF16S * 16 + 8: return launch_v2<LBM_STORE_BF16S, 8>(P, overlap, s);
-    case LBM_STORE_F16R * 16 + 4: return launch_v2<LBM_STORE_F16S, 4, true>(P, overlap, s);
-    case LBM_STORE_BF16R * 16 + 4: return launch_v2<LBM_STORE_BF16S, 4, true>(P, overlap, s);
-    default: return dispatch<MODE_FUSED>(storage, flags & LBM_FLAG_EXACT, P, s);
   }
 }
 
@@ -522,6 +563,7 @@ int lbm_lattice_run_opts(const lbm_geometry* g, int32_t storage, void* pop_a, vo
   P.pop_out = pop_b;
   P.aux_in = aux_a;
   P.aux_out = aux_b;
+  if (storage == LBM_STORE_FX64 && v2_npt(storage, flags, P) > 0) set_fx_tables(P.g);
   const int tiled_steps = nsteps - (rho_out != nullptr || u_out != nullptr ? 1 : 0);
   TilePlan plan;
   if (tiled_steps >= 3 && tile_applies(storage, flags, P)) plan = tile_plan(storage, P);

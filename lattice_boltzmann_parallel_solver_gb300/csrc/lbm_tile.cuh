@@ -157,10 +157,13 @@ __device__ __forceinline__ void tile_body(const KParams& P, const void* pop_in_v
     }
     for (int j = tid; j < 9 * LBM_MAX_SETS; j += nthr) {
       const int set = j / 9, i = j - 9 * set;
-      const double kc = P.g.kconst[set][i], cc = P.g.cconst[set][i];
-      if constexpr (FX) skc[j] = fx::round_scaled(kc, fx::kS);
-      else skc[j] = (R)kc * kS;
-      scc[j] = work_of_f((R)cc, i);
+      if constexpr (FX) {  // fixed point already (set_fx_tables)
+        skc[j] = __double_as_longlong(P.g.kconst[set][i]);
+        scc[j] = __double_as_longlong(P.g.cconst[set][i]);
+      } else {
+        skc[j] = (R)P.g.kconst[set][i] * kS;
+        scc[j] = work_of_f((R)P.g.cconst[set][i], i);
+      }
     }
     // tiles away from every boundary skip the sources altogether
     any_bc = __syncthreads_or(any_bc);

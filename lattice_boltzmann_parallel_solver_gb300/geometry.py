@@ -104,6 +104,7 @@ class CompiledGeometry:
             g.bcnodes = self.bcnodes.data_ptr()
             g.n_bcnodes = int(order.size)
             g.n_bcnodes_edge = int(edge.sum())
+            self._frame(g, nx, ny, nodes, desc.reshape(ny, nx))
             g.n_kset, g.n_cset = len(ktab), len(ctab)
             for s_ in range(len(ktab)):
                 for i in range(9):
@@ -122,6 +123,31 @@ class CompiledGeometry:
             assert nx >= 2
         self.pressure = pressure
         self.struct = g
+
+    @staticmethod
+    def _frame(g, nx, ny, nodes, desc):
+        """Sets the frame: the one descriptor of each side (without its corners)
+        and of each corner, and the box of the other boundary nodes (``nodes``).
+        Left unset when a side mixes descriptors or only some of its nodes have
+        one.  ``desc``: the descriptors [ny, nx]."""
+        if nx < 3 or ny < 3:
+            return
+        sides = (desc[0, 1:-1], desc[-1, 1:-1], desc[1:-1, 0], desc[1:-1, -1])
+        descs = [int(side[0]) for side in sides]
+        if any((side != d).any() for side, d in zip(sides, descs)):
+            return
+        on_frame = sum(side.size for side, d in zip(sides, descs) if d)
+        descs += [int(desc[0, 0]), int(desc[0, -1]), int(desc[-1, 0]), int(desc[-1, -1])]
+        on_frame += sum(d != 0 for d in descs[4:])
+        box = (1, 0, 1, 0)
+        if nodes.size > on_frame:
+            x, y = nodes % nx, nodes // nx
+            inner = (x > 0) & (x < nx - 1) & (y > 0) & (y < ny - 1)
+            x, y = x[inner], y[inner]
+            box = (int(x.min()), int(x.max()), int(y.min()), int(y.max()))
+        g.frame = 1
+        g.frame_desc[:] = descs
+        g.inner_box[:] = box
 
     @staticmethod
     def _edge_desc(nx, ny, nodes, src, packed, edge):

@@ -72,11 +72,12 @@ class Lattice:
         ``stochastic`` (default: on for the 16-bit storages) rounds the stored
         deviations stochastically, which keeps increments smaller than half a
         16-bit step from being lost; ``seed`` seeds its random bits.
-        Large lattices (from 2^22 nodes in the 16-bit storages, 2^25 in the
-        others) run the vectorised step without boundary work and then a pass
-        over the boundary nodes; smaller ones apply the boundary sources inside
-        the step (same results).  ``bc_inline`` True / False forces the one or
-        the other.  The
+        In "f32" (in the other storages from 2^25 nodes) the vectorised step
+        leaves the boundary nodes to a pass over them; else it applies the
+        boundary sources inside (same results).  ``bc_inline`` True / False
+        forces the one or the other.  Small lattices (up to a few hundred
+        thousand nodes) take several steps per launch (same results);
+        ``bc_inline``, ``npt``, ``generic`` and ``exact`` keep one.  The
         default storage is "fx64", or "f64" with ``exact`` (the reference's
         float64 operation order, bit for bit).  ``probe`` = (x, y) records the
         velocity of that node at every fused step, up to ``probe_cap`` steps

@@ -11,8 +11,6 @@
 
 namespace lbm {
 
-enum { MODE_INIT = 0, MODE_FUSED = 1, MODE_READ = 2 };
-
 struct GeoK {
   int nx, ny, words;
   const uint32_t* bcmask;
@@ -39,10 +37,6 @@ struct GeoK {
 };
 
 
-struct View {
-  const double* p;
-  int64_t sx, sy, sc;
-};
 struct OutView {
   double* p;
   int64_t sx, sy, sc;
@@ -50,15 +44,14 @@ struct OutView {
 
 struct KParams {
   GeoK g;
-  // columns [xb, xe) handled by the one-node-per-thread kernel (xe == 0: all)
+  // columns [xb, xe) handled by the init and read kernels (xe == 0: all)
   int xb, xe;
   const void* pop_in;
   void* pop_out;
   int64_t pitch, plane;
   const void* aux_in;
   void* aux_out;
-  View f_in, rho_in, u_in;
-  OutView f_out, rho_out, u_out;
+  OutView rho_out, u_out;
   double omega;
   // optional probe: the fused step at node (probe_x, probe_y) appends its
   // pre-collision velocity to probe_buf[2 * t], t = (*probe_count)++
@@ -806,14 +799,14 @@ struct __align__(16) BatchEntry {
 // that one drains.  The first launch of a run stays a plain one: it may follow
 // any kernel of the caller's, also one that writes the geometry.
 template <typename... Params, typename... Args>
-inline void launch_step(void (*kernel)(Params...), dim3 grid, int threads, bool overlap, cudaStream_t s, size_t smem,
+inline void launch_step(void (*kernel)(Params...), dim3 grid, dim3 block, bool overlap, cudaStream_t s, size_t smem,
                         const Args&... args) {
   cudaLaunchAttribute at = {};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c = {};
   c.gridDim = grid;
-  c.blockDim = dim3((unsigned)threads);
+  c.blockDim = block;
   c.dynamicSmemBytes = smem;
   c.stream = s;
   c.attrs = &at;

@@ -8,14 +8,15 @@
 // kernel per step reads S_{n-1} once (pull: node x takes S(x - c_i, i)),
 // applies the boundary sources, forms the moments of f_n, collides and
 // writes S_n once: 72 B read + 72 B written per node in float64.
-//   MODE_INIT  : S_0 = collide(f_0) from a reference-layout f_0 (rho,u passed in or recomputed)
-//   MODE_FUSED : S_n from S_{n-1}
-//   MODE_READ  : f_n = BC(stream(S_{n-1})) and its moments, in the reference layout
+//   init_kernel : S_0 = collide(f_0) from a reference-layout f_0 (rho,u passed in or recomputed)
+//   the steps   : S_n from S_{n-1}
+//   read_kernel : f_n = BC(stream(S_{n-1})) and its moments, in the reference layout
 // The outlet (boundary_conditions.py:279-280) needs f_{n-1} at column nx-2;
 // each kernel stores those three populations in aux[3][ny] for the next one.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "lbm_fused.cuh"
@@ -23,122 +24,91 @@
 
 namespace lbm {
 
-template <int STORE, bool EXACT, int MODE>
-__global__ void __launch_bounds__(256) lattice_kernel(const __grid_constant__ KParams P) {
+// The generic one-node-per-thread code: any geometry, any storage, exact or FMA
+// arithmetic.
+
+// populations of a storage as the generic code reads and writes them: in the
+// reference-shifted 16-bit storages (dev_shift) the stored deviation is taken
+// from c_i = w_i + sig_i instead of w_i
+template <int STORE>
+__device__ __forceinline__ typename Store<STORE>::R node_ld(const KParams& P, const typename Store<STORE>::T* p, int i) {
+  using R = typename Store<STORE>::R;
+  const R v = Store<STORE>::ld(p, i);
+  if constexpr (Store<STORE>::kShifted) return P.dev_shift ? v + (R)P.shf[1].sig[i] : v;
+  else return v;
+}
+template <int STORE>
+__device__ __forceinline__ void node_st(const KParams& P, typename Store<STORE>::T* p, typename Store<STORE>::R v, int i) {
+  using R = typename Store<STORE>::R;
+  if constexpr (Store<STORE>::kShifted) Store<STORE>::st(p, P.dev_shift ? v - (R)P.shf[1].sig[i] : v, i);
+  else Store<STORE>::st(p, v, i);
+}
+
+// f of node (x, y) pulled from the collided populations, with its boundary sources
+template <int STORE, bool EXACT>
+__device__ __forceinline__ void pull_node(const KParams& P, int x, int y, typename Store<STORE>::R f[9]) {
   using St = Store<STORE>;
   using T = typename St::T;
   using R = typename St::R;
   const int nx = P.g.nx, ny = P.g.ny;
-  const int x = P.xb + blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= (P.xe > 0 ? P.xe : nx) || y >= ny) return;
   const int64_t r0 = (int64_t)y * P.pitch;
-  using A = typename St::A;
-  const A* aux_in = static_cast<const A*>(P.aux_in);
-  // reference-shifted 16-bit storages: the stored deviation is taken from
-  // c_i = w_i + sig_i instead of w_i
-  const bool shift = St::kShifted && P.dev_shift;
-  auto ld = [&](const T* p, int i) -> R {
-    const R v = St::ld(p, i);
-    if constexpr (St::kShifted) return shift ? v + (R)P.shf[1].sig[i] : v;
-    else return v;
-  };
-  auto st = [&](T* p, R v, int i) {
-    if constexpr (St::kShifted) St::st(p, shift ? v - (R)P.shf[1].sig[i] : v, i);
-    else St::st(p, v, i);
-  };
-
-  R f[9];
-  if (MODE == MODE_INIT) {
-    const double* src = P.f_in.p + x * P.f_in.sx + y * P.f_in.sy;
-#pragma unroll
-    for (int i = 0; i < 9; ++i) f[i] = (R)src[i * P.f_in.sc];
-  } else {
-    // pull: direction i arrives from node (x - cx_i, y - cy_i), periodic
-    const int xm = x == 0 ? nx - 1 : x - 1, xp = x == nx - 1 ? 0 : x + 1;
-    const int ym = y == 0 ? ny - 1 : y - 1, yp = y == ny - 1 ? 0 : y + 1;
-    const int64_t rm = (int64_t)ym * P.pitch, rp = (int64_t)yp * P.pitch;
-    const T* pin = static_cast<const T*>(P.pop_in);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      const int xs = cx(i) == 1 ? xm : (cx(i) == -1 ? xp : x);
-      const int64_t rs = cy(i) == 1 ? rm : (cy(i) == -1 ? rp : r0);
-      f[i] = ld(pin + i * P.plane + rs + xs, i);
-    }
-    if (P.g.bcmask != nullptr) {
-      const uint32_t word = __ldg(P.g.bcmask + (int64_t)y * P.g.words + (x >> 5));
-      if ((word >> (x & 31)) & 1u) {
-        const uint32_t d = __ldg(P.g.desc + (int64_t)y * nx + x);
-        const int ks = (d >> LBM_DESC_KSET_SHIFT) & 15, cs = (d >> LBM_DESC_CSET_SHIFT) & 15;
-#pragma unroll
-        for (int i = 0; i < 9; ++i) {
-          const uint32_t s = (d >> (2 * i)) & 3u;
-          if (s == LBM_SRC_BOUNCE) {
-            const R v = ld(pin + opp(i) * P.plane + r0 + x, opp(i));
-            if (EXACT)
-              f[i] = (R)__dsub_rn((double)v, P.g.kconst[ks][i]);
-            else
-              f[i] = v - (R)P.g.kconst[ks][i];
-          } else if (s == LBM_SRC_CONST) {
-            f[i] = (R)P.g.cconst[cs][i];
-          } else if (s == LBM_SRC_OUTLET && outlet_slot(i) >= 0 && aux_in != nullptr) {
-            f[i] = St::from_aux(aux_in[outlet_slot(i) * ny + y], i);
+  const typename St::A* aux_in = static_cast<const typename St::A*>(P.aux_in);
+  auto ld = [&](const T* p, int i) -> R { return node_ld<STORE>(P, p, i); };
+      // pull: direction i arrives from node (x - cx_i, y - cy_i), periodic
+      const int xm = x == 0 ? nx - 1 : x - 1, xp = x == nx - 1 ? 0 : x + 1;
+      const int ym = y == 0 ? ny - 1 : y - 1, yp = y == ny - 1 ? 0 : y + 1;
+      const int64_t rm = (int64_t)ym * P.pitch, rp = (int64_t)yp * P.pitch;
+      const T* pin = static_cast<const T*>(P.pop_in);
+  #pragma unroll
+      for (int i = 0; i < 9; ++i) {
+        const int xs = cx(i) == 1 ? xm : (cx(i) == -1 ? xp : x);
+        const int64_t rs = cy(i) == 1 ? rm : (cy(i) == -1 ? rp : r0);
+        f[i] = ld(pin + i * P.plane + rs + xs, i);
+      }
+      if (P.g.bcmask != nullptr) {
+        const uint32_t word = __ldg(P.g.bcmask + (int64_t)y * P.g.words + (x >> 5));
+        if ((word >> (x & 31)) & 1u) {
+          const uint32_t d = __ldg(P.g.desc + (int64_t)y * nx + x);
+          const int ks = (d >> LBM_DESC_KSET_SHIFT) & 15, cs = (d >> LBM_DESC_CSET_SHIFT) & 15;
+  #pragma unroll
+          for (int i = 0; i < 9; ++i) {
+            const uint32_t s = (d >> (2 * i)) & 3u;
+            if (s == LBM_SRC_BOUNCE) {
+              const R v = ld(pin + opp(i) * P.plane + r0 + x, opp(i));
+              if (EXACT)
+                f[i] = (R)__dsub_rn((double)v, P.g.kconst[ks][i]);
+              else
+                f[i] = v - (R)P.g.kconst[ks][i];
+            } else if (s == LBM_SRC_CONST) {
+              f[i] = (R)P.g.cconst[cs][i];
+            } else if (s == LBM_SRC_OUTLET && outlet_slot(i) >= 0 && aux_in != nullptr) {
+              f[i] = St::from_aux(aux_in[outlet_slot(i) * ny + y], i);
+            }
           }
         }
       }
-    }
-  }
+}
 
+// Collides node (x, y) of f_n in place (its moments rho, ux, uy as given) and
+// stores S_n and the outlet memory.
+template <int STORE, bool EXACT>
+__device__ __forceinline__ void collide_store(const KParams& P, int x, int y, typename Store<STORE>::R f[9],
+                                              typename Store<STORE>::R rho, typename Store<STORE>::R ux,
+                                              typename Store<STORE>::R uy) {
+  using St = Store<STORE>;
+  using T = typename St::T;
+  using R = typename St::R;
+  using A = typename St::A;
+  const int nx = P.g.nx, ny = P.g.ny;
+  const int64_t r0 = (int64_t)y * P.pitch;
+  auto st = [&](T* p, R v, int i) { node_st<STORE>(P, p, v, i); };
   // outlet memory: the pre-collision populations 3,6,7 of column nx-2
-  if (MODE != MODE_READ && P.aux_out != nullptr && x == nx - 2) {
+  if (P.aux_out != nullptr && x == nx - 2) {
     A* aux_out = static_cast<A*>(P.aux_out);
     aux_out[0 * ny + y] = St::to_aux(f[3], 3);
     aux_out[1 * ny + y] = St::to_aux(f[6], 6);
     aux_out[2 * ny + y] = St::to_aux(f[7], 7);
   }
-
-  // moments of f_n; the collision of the first step uses the rho,u passed in
-  R rho, ux, uy;
-  const bool given = MODE == MODE_INIT && P.rho_in.p != nullptr;
-  if (given) {
-    rho = (R)P.rho_in.p[x * P.rho_in.sx + y * P.rho_in.sy];
-    const double* up = P.u_in.p + x * P.u_in.sx + y * P.u_in.sy;
-    ux = (R)up[0];
-    uy = (R)up[P.u_in.sc];
-  } else if (EXACT || MODE == MODE_READ) {
-    // read-out moments always follow compute_density / compute_velocity_field exactly
-    double fd[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) fd[i] = (double)f[i];
-    const double r = density9_exact(fd);
-    double a, b;
-    velocity_exact(fd, r, a, b);
-    rho = (R)r;
-    ux = (R)a;
-    uy = (R)b;
-  } else {
-    rho = density9(f);
-    velocity_fast(f, rho, ux, uy);
-  }
-
-  if (MODE == MODE_FUSED) write_probe(P, x, y, ux, uy);
-  if (MODE == MODE_READ || (MODE == MODE_FUSED && P.rho_out.p != nullptr)) {
-    if (P.rho_out.p != nullptr) P.rho_out.p[x * P.rho_out.sx + y * P.rho_out.sy] = (double)rho;
-    if (P.u_out.p != nullptr) {
-      double* up = P.u_out.p + x * P.u_out.sx + y * P.u_out.sy;
-      up[0] = (double)ux;
-      up[P.u_out.sc] = (double)uy;
-    }
-  }
-  if (MODE == MODE_READ) {
-    if (P.f_out.p != nullptr) {
-      double* dst = P.f_out.p + x * P.f_out.sx + y * P.f_out.sy;
-#pragma unroll
-      for (int i = 0; i < 9; ++i) dst[i * P.f_out.sc] = (double)f[i];
-    }
-    return;
-  }
-
   // collision
   const bool pressure_src = P.g.pressure && (x == nx - 2 || x == 1);
   R pin_v[9], pout_v[9];
@@ -187,6 +157,149 @@ __global__ void __launch_bounds__(256) lattice_kernel(const __grid_constant__ KP
 #pragma unroll
       for (int i = 0; i < 9; ++i)
         if ((P.g.pout >> i) & 1u) st(pout + i * P.plane + r0 + (nx - 1), pout_v[i], i);
+    }
+  }
+}
+
+// moments of f_n: exactly as compute_density / compute_velocity_field, or the FMA form
+template <bool EXACT, typename R>
+__device__ __forceinline__ void node_moments(const R f[9], R& rho, R& ux, R& uy) {
+  if constexpr (EXACT) {
+    double fd[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) fd[i] = (double)f[i];
+    const double r = density9_exact(fd);
+    double a, b;
+    velocity_exact(fd, r, a, b);
+    rho = (R)r;
+    ux = (R)a;
+    uy = (R)b;
+  } else {
+    rho = density9(f);
+    velocity_fast(f, rho, ux, uy);
+  }
+}
+
+// S_n from S_{n-1}, one node per thread
+template <int STORE, bool EXACT>
+__global__ void __launch_bounds__(256) lattice_kernel(const __grid_constant__ KParams P) {
+  using R = typename Store<STORE>::R;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+  if (x >= P.g.nx || y >= P.g.ny) return;
+  R f[9], rho, ux, uy;
+  pull_node<STORE, EXACT>(P, x, y, f);
+  node_moments<EXACT>(f, rho, ux, uy);
+  write_probe(P, x, y, ux, uy);
+  if (P.rho_out.p != nullptr) {
+    P.rho_out.p[x * P.rho_out.sx + y * P.rho_out.sy] = (double)rho;
+    if (P.u_out.p != nullptr) {
+      double* up = P.u_out.p + x * P.u_out.sx + y * P.u_out.sy;
+      up[0] = (double)ux;
+      up[P.u_out.sc] = (double)uy;
+    }
+  }
+  collide_store<STORE, EXACT>(P, x, y, f, rho, ux, uy);
+}
+
+// The read-out goes from the resident layout (x fastest) to the reference's
+// f[x][y][9] (y fastest).  In the 64-bit storages a tile of kTileX x kTileY nodes
+// passes through shared memory, so that both sides move whole runs (32 elements of
+// a plane per row, 576 B of f per column of the tile; a thread that stores its
+// node's 72 B itself takes a sector per population).  The shared rows are 73, 9 and
+// 17 doubles long: odd, so that lanes along x hit different banks.  What is left is
+// float64 arithmetic, some 40 instructions a node (conversions, exact moments with
+// two divisions) on a pipe that serves 1.6 a clock per SM.  1024^2 with f, us: f64
+// 130 -> 98, fx64 147 -> 128.  The float32 and 16-bit storages are bound by it
+// already (128 either way, and the barrier costs small lattices 2 us), so a thread
+// writes its node there.  (The first step through shared memory lost, 150 -> 164 us
+// in float64: its loads wait for nobody as they are, and the barrier made the
+// float64 work wait for them.)
+constexpr int kTileX = 32, kTileY = 8, kTileThreads = kTileX * kTileY;
+struct RefTile {
+  double f[kTileX][9 * kTileY + 1];
+  double rho[kTileX][kTileY + 1];
+  double u[kTileX][2 * kTileY + 1];
+};
+
+// Writes the shared tile to the reference layout (N values per node); columns
+// x0 .. xe - 1, rows y0 .. ny - 1 at most.
+template <int N, int W>
+__device__ __forceinline__ void tile_write(double* g, const double (*s)[W], int tid, int x0, int xe, int y0,
+                                           int ny) {
+  static_assert(W == N * kTileY + 1, "a tile column and one more");
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const int e = tid + j * kTileThreads, c = e / (N * kTileY), r = e - c * (N * kTileY);
+    if (x0 + c < xe && y0 + r / N < ny) g[((int64_t)(x0 + c) * ny + y0) * N + r] = s[c][r];
+  }
+}
+
+// S_0 = collide(f_0) from the reference layout, with the rho, u passed in or their moments
+template <int STORE, bool EXACT>
+__global__ void __launch_bounds__(256) init_kernel(const __grid_constant__ KParams P, const double* f_in,
+                                                   const double* rho_in, const double* u_in) {
+  using R = typename Store<STORE>::R;
+  const int ny = P.g.ny, x = P.xb + blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+  if (x >= (P.xe > 0 ? P.xe : P.g.nx) || y >= ny) return;
+  const int64_t n = (int64_t)x * ny + y;
+  R f[9], rho, ux, uy;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) f[i] = (R)f_in[9 * n + i];
+  if (rho_in != nullptr) {
+    rho = (R)rho_in[n];
+    ux = (R)u_in[2 * n];
+    uy = (R)u_in[2 * n + 1];
+  } else {
+    node_moments<EXACT>(f, rho, ux, uy);
+  }
+  collide_store<STORE, EXACT>(P, x, y, f, rho, ux, uy);
+}
+
+template <int STORE>
+constexpr bool read_tiled() { return sizeof(typename Store<STORE>::T) == 8; }
+
+// f_n = BC(stream(S_{n-1})) and its moments in the reference layout (each of the
+// outputs may be null); the moments always follow compute_density /
+// compute_velocity_field exactly.  Blocks of kTileX x kTileY threads in the tiled
+// form, of node_grid otherwise.
+template <int STORE, bool EXACT>
+__global__ void __launch_bounds__(256) read_kernel(const __grid_constant__ KParams P, double* f_out, double* rho_out,
+                                                   double* u_out) {
+  using R = typename Store<STORE>::R;
+  pdl_wait();
+  const int ny = P.g.ny, xe = P.xe > 0 ? P.xe : P.g.nx;
+  const int x0 = P.xb + (int)(blockIdx.x * blockDim.x), y0 = (int)(blockIdx.y * blockDim.y);
+  const int c = (int)threadIdx.x, r = (int)threadIdx.y, x = x0 + c, y = y0 + r;
+  R f[9], rho, ux, uy;
+  const bool in = x < xe && y < ny;
+  if (in) {
+    pull_node<STORE, EXACT>(P, x, y, f);
+    node_moments<true>(f, rho, ux, uy);
+  }
+  if constexpr (read_tiled<STORE>()) {
+    __shared__ RefTile t;
+    if (in) {
+#pragma unroll
+      for (int i = 0; i < 9; ++i) t.f[c][9 * r + i] = (double)f[i];
+      t.rho[c][r] = (double)rho;
+      t.u[c][2 * r] = (double)ux;
+      t.u[c][2 * r + 1] = (double)uy;
+    }
+    __syncthreads();
+    const int tid = r * kTileX + c;
+    if (f_out != nullptr) tile_write<9>(f_out, t.f, tid, x0, xe, y0, ny);
+    if (rho_out != nullptr) tile_write<1>(rho_out, t.rho, tid, x0, xe, y0, ny);
+    if (u_out != nullptr) tile_write<2>(u_out, t.u, tid, x0, xe, y0, ny);
+  } else if (in) {
+    const int64_t n = (int64_t)x * ny + y;
+    if (rho_out != nullptr) rho_out[n] = (double)rho;
+    if (u_out != nullptr) {
+      u_out[2 * n] = (double)ux;
+      u_out[2 * n + 1] = (double)uy;
+    }
+    if (f_out != nullptr) {
+#pragma unroll
+      for (int i = 0; i < 9; ++i) f_out[9 * n + i] = (double)f[i];
     }
   }
 }
@@ -271,42 +384,75 @@ __global__ void advance_counter_kernel(int32_t* counter, int32_t n) { *counter +
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-static void launch_dims(int nx, int ny, dim3& grid, dim3& block) {
-  int bx = nx >= 128 ? 128 : ((nx + 31) / 32) * 32;
-  int by = std::max(1, 128 / bx);
-  block = dim3(bx, by, 1);
-  grid = dim3((nx + bx - 1) / bx, (ny + by - 1) / by, 1);
-}
-
-template <int STORE, bool EXACT, int MODE>
-static int launch(const KParams& P, cudaStream_t s) {
-  dim3 grid, block;
-  launch_dims((P.xe > 0 ? P.xe : P.g.nx) - P.xb, P.g.ny, grid, block);
-  lattice_kernel<STORE, EXACT, MODE><<<grid, block, 0, s>>>(P);
-  count_launch();
-  return check_launch("lattice_kernel");
-}
-
-template <int MODE>
-static int dispatch(int storage, bool exact, const KParams& P, cudaStream_t s) {
+// f(storage, exact) with the storage and the arithmetic as compile-time numbers
+template <typename F>
+static int by_storage(int storage, bool exact, const KParams& P, F&& f) {
   if (exact && storage != LBM_STORE_F64)
     return set_error(LBM_ERR_UNSUPPORTED, "exact arithmetic needs float64 storage");
+  using std::integral_constant;
+  constexpr std::false_type fma{};
   switch (storage) {
     case LBM_STORE_F64:
-      return exact ? launch<LBM_STORE_F64, true, MODE>(P, s) : launch<LBM_STORE_F64, false, MODE>(P, s);
-    case LBM_STORE_F32: return launch<LBM_STORE_F32, false, MODE>(P, s);
-    case LBM_STORE_F16S: return launch<LBM_STORE_F16S, false, MODE>(P, s);
-    case LBM_STORE_BF16S: return launch<LBM_STORE_BF16S, false, MODE>(P, s);
-    case LBM_STORE_FX64: return launch<LBM_STORE_FX64, false, MODE>(P, s);
+      return exact ? f(P, integral_constant<int, LBM_STORE_F64>{}, std::true_type{})
+                   : f(P, integral_constant<int, LBM_STORE_F64>{}, fma);
+    case LBM_STORE_F32: return f(P, integral_constant<int, LBM_STORE_F32>{}, fma);
+    case LBM_STORE_F16S: return f(P, integral_constant<int, LBM_STORE_F16S>{}, fma);
+    case LBM_STORE_BF16S: return f(P, integral_constant<int, LBM_STORE_BF16S>{}, fma);
+    case LBM_STORE_FX64: return f(P, integral_constant<int, LBM_STORE_FX64>{}, fma);
     case LBM_STORE_F16R:
     case LBM_STORE_BF16R: {
       KParams Q = P;
       Q.dev_shift = 1;
-      return storage == LBM_STORE_F16R ? launch<LBM_STORE_F16S, false, MODE>(Q, s)
-                                       : launch<LBM_STORE_BF16S, false, MODE>(Q, s);
+      return storage == LBM_STORE_F16R ? f(Q, integral_constant<int, LBM_STORE_F16S>{}, fma)
+                                       : f(Q, integral_constant<int, LBM_STORE_BF16S>{}, fma);
     }
     default: return set_error(LBM_ERR_ARG, "unknown storage type");
   }
+}
+
+// one thread per node, along x
+static void node_grid(int w, int ny, dim3& grid, dim3& block) {
+  const int bx = w >= 128 ? 128 : (w + 31) / 32 * 32, by = std::max(1, 128 / bx);
+  block = dim3((unsigned)bx, (unsigned)by);
+  grid = dim3((unsigned)((w + bx - 1) / bx), (unsigned)((ny + by - 1) / by));
+}
+
+// one generic step
+static int launch_node(int storage, bool exact, const KParams& P, cudaStream_t s) {
+  return by_storage(storage, exact, P, [&](const KParams& Q, auto store, auto ex) {
+    dim3 grid, block;
+    node_grid(Q.g.nx, Q.g.ny, grid, block);
+    lattice_kernel<store(), ex()><<<grid, block, 0, s>>>(Q);
+    count_launch();
+    return check_launch("lattice_kernel");
+  });
+}
+
+static int launch_init(int storage, bool exact, const KParams& P, const double* f, const double* rho, const double* u,
+                       cudaStream_t s) {
+  return by_storage(storage, exact, P, [&](const KParams& Q, auto store, auto ex) {
+    dim3 grid, block;
+    node_grid((Q.xe > 0 ? Q.xe : Q.g.nx) - Q.xb, Q.g.ny, grid, block);
+    init_kernel<store(), ex()><<<grid, block, 0, s>>>(Q, f, rho, u);
+    count_launch();
+    return check_launch("init_kernel");
+  });
+}
+
+// `overlap`: right after the init_kernel of the same call
+static int launch_read(int storage, bool exact, const KParams& P, double* f, double* rho, double* u, bool overlap,
+                       cudaStream_t s) {
+  return by_storage(storage, exact, P, [&](const KParams& Q, auto store, auto ex) {
+    const int w = (Q.xe > 0 ? Q.xe : Q.g.nx) - Q.xb;
+    dim3 grid, block(kTileX, kTileY);
+    if (read_tiled<store()>())
+      grid = dim3((unsigned)((w + kTileX - 1) / kTileX), (unsigned)((Q.g.ny + kTileY - 1) / kTileY));
+    else
+      node_grid(w, Q.g.ny, grid, block);
+    launch_step(read_kernel<store(), ex()>, grid, block, overlap, s, 0, Q, f, rho, u);
+    count_launch();
+    return check_launch("read_kernel");
+  });
 }
 
 constexpr int kV2Threads = 128;
@@ -416,7 +562,7 @@ static int launch_fused_step(int storage, int npt, int bc, int flags, const KPar
     case LBM_STORE_BF16S * 16 + 8: return launch_v2<LBM_STORE_BF16S, 8>(P, bc, overlap, s);
     case LBM_STORE_F16R * 16 + 4: return launch_v2<LBM_STORE_F16S, 4, true>(P, bc, overlap, s);
     case LBM_STORE_BF16R * 16 + 4: return launch_v2<LBM_STORE_BF16S, 4, true>(P, bc, overlap, s);
-    default: return dispatch<MODE_FUSED>(storage, flags & LBM_FLAG_EXACT, P, s);
+    default: return launch_node(storage, flags & LBM_FLAG_EXACT, P, s);
   }
 }
 
@@ -473,13 +619,6 @@ static size_t store_bytes(int storage) {
   }
 }
 
-static View ref_f(const double* p, int ny) { return View{p, 9LL * ny, 9, 1}; }
-static View ref_rho(const double* p, int ny) { return View{p, (int64_t)ny, 1, 0}; }
-static View ref_u(const double* p, int ny) { return View{p, 2LL * ny, 2, 1}; }
-static OutView ref_f_out(double* p, int ny) { return OutView{p, 9LL * ny, 9, 1}; }
-static OutView ref_rho_out(double* p, int ny) { return OutView{p, (int64_t)ny, 1, 0}; }
-static OutView ref_u_out(double* p, int ny) { return OutView{p, 2LL * ny, 2, 1}; }
-
 }  // namespace lbm
 
 using namespace lbm;
@@ -506,14 +645,9 @@ int lbm_lattice_init(const lbm_geometry* g, int32_t storage, const double* f, co
   P.pitch = pitch;
   P.plane = pitch * g->ny;
   P.aux_out = aux_out;
-  P.f_in = ref_f(f, g->ny);
-  if (rho) {
-    P.rho_in = ref_rho(rho, g->ny);
-    P.u_in = ref_u(u, g->ny);
-  }
   P.omega = omega;
   set_shift(P);
-  return dispatch<MODE_INIT>(storage, flags & LBM_FLAG_EXACT, P, (cudaStream_t)stream);
+  return launch_init(storage, flags & LBM_FLAG_EXACT, P, f, rho, u, (cudaStream_t)stream);
 }
 
 int lbm_lattice_run(const lbm_geometry* g, int32_t storage, void* pop_a, void* pop_b, int64_t pitch,
@@ -614,11 +748,8 @@ int lbm_lattice_read(const lbm_geometry* g, int32_t storage, const void* pop, in
   P.aux_in = aux;
   P.pitch = pitch;
   P.plane = pitch * g->ny;
-  P.f_out = ref_f_out(f_out, g->ny);
-  P.rho_out = ref_rho_out(rho_out, g->ny);
-  P.u_out = ref_u_out(u_out, g->ny);
   set_shift(P);  // omega 1: the read converts, it does not collide
-  return dispatch<MODE_READ>(storage, false, P, (cudaStream_t)stream);
+  return launch_read(storage, false, P, f_out, rho_out, u_out, false, (cudaStream_t)stream);
 }
 
 size_t lbm_step_scratch_bytes(int32_t nx, int32_t ny) {
@@ -645,11 +776,7 @@ int lbm_step_f64(const lbm_geometry* g, const double* f, const double* rho, cons
   P.aux_in = aux;
   P.pitch = pitch;
   P.plane = pitch * g->ny;
-  P.f_out = ref_f_out(f_out, g->ny);
-  P.rho_out = ref_rho_out(rho_out, g->ny);
-  P.u_out = ref_u_out(u_out, g->ny);
-  return (flags & LBM_FLAG_EXACT) ? launch<LBM_STORE_F64, true, MODE_READ>(P, (cudaStream_t)stream)
-                                  : launch<LBM_STORE_F64, false, MODE_READ>(P, (cudaStream_t)stream);
+  return launch_read(LBM_STORE_F64, flags & LBM_FLAG_EXACT, P, f_out, rho_out, u_out, true, (cudaStream_t)stream);
 }
 
 // ---- the drop-in step on host buffers, with copies and kernels overlapped ----
@@ -728,12 +855,9 @@ int lbm_step_f64_host(const lbm_geometry* g, const double* f, const double* rho,
     P.pitch = pitch;
     P.plane = pitch * ny;
     P.aux_out = aux;
-    P.f_in = ref_f(fin, ny);
-    P.rho_in = ref_rho(rin, ny);
-    P.u_in = ref_u(uin, ny);
     P.omega = omega;
     if (!cuda_ok(cudaStreamWaitEvent(sc, in_ready[k], 0))) return;
-    const int e = exact ? launch<LBM_STORE_F64, true, MODE_INIT>(P, sc) : launch<LBM_STORE_F64, false, MODE_INIT>(P, sc);
+    const int e = launch_init(LBM_STORE_F64, exact, P, fin, rin, uin, sc);
     if (e != LBM_OK && st == LBM_OK) st = e;
   };
   auto read = [&](int k) {
@@ -745,10 +869,7 @@ int lbm_step_f64_host(const lbm_geometry* g, const double* f, const double* rho,
     P.aux_in = aux;
     P.pitch = pitch;
     P.plane = pitch * ny;
-    P.f_out = ref_f_out(fo, ny);
-    P.rho_out = ref_rho_out(ro, ny);
-    P.u_out = ref_u_out(uo, ny);
-    const int e = exact ? launch<LBM_STORE_F64, true, MODE_READ>(P, sc) : launch<LBM_STORE_F64, false, MODE_READ>(P, sc);
+    const int e = launch_read(LBM_STORE_F64, exact, P, fo, ro, uo, false, sc);
     if (e != LBM_OK && st == LBM_OK) st = e;
     out_ready[k] = event();
     cuda_ok(cudaEventRecord(out_ready[k], sc));

@@ -26,6 +26,7 @@ int lbm_batch_build(const lbm_batch_lattice* lat, int32_t n, int32_t npt, int32_
   int64_t tiles = 0, chunks_bc = 0, nodes = 0;
   bool inline_bc = false;  // some lattice has boundary nodes but no list of them
   bool force_split = false;
+  bool wide_box = false;  // some lattice's boundary nodes are spread over it
   for (int j = 0; j < n; ++j) {
     const lbm_batch_lattice& L = lat[j];
     BatchEntry& e = ent[(size_t)j];
@@ -65,11 +66,12 @@ int lbm_batch_build(const lbm_batch_lattice* lat, int32_t n, int32_t npt, int32_
     e.rows = L.rows > 0 ? L.rows : 1;
     if (e.P.g.bcmask != nullptr && (e.P.g.n_bcnodes == 0 || (L.flags & LBM_FLAG_BC_INLINE))) inline_bc = true;
     if (L.flags & LBM_FLAG_BC_SPLIT) force_split = true;
+    if (e.P.g.bcmask != nullptr && !small_box(e.P.g)) wide_box = true;
     nodes += (int64_t)L.g->nx * L.g->ny;
     bc_start[(size_t)j] = (int)chunks_bc;
     chunks_bc += (pass_nodes(e.P.g) + threads - 1) / threads;
   }
-  if (nodes < kBatchPassNodes && !force_split) inline_bc = true;
+  if ((nodes < kBatchPassNodes || (nodes < kBatchSplitNodes && wide_box)) && !force_split) inline_bc = true;
   // tiles: runs across row ends with the pass, row segments without it
   for (int j = 0; j < n; ++j) {
     const BatchEntry& e = ent[(size_t)j];

@@ -928,6 +928,15 @@ inline void set_fx_tables(GeoK& g) {
   for (int i = 0; i < 9; ++i) put(g.edge_in_f[i], fx::to_fx(g.edge_in_f[i], wd(i)));
 }
 
+// Whether a body that leaves the boundary nodes out finds them cheaply: chunks in
+// the inner box read the mask and store node by node, so the box may hold an
+// eighth of the lattice at most (obstacles all over it, or sides that mix
+// descriptors and so have no frame, keep the sources inside the body)
+inline bool small_box(const GeoK& g) {
+  const int64_t w = std::max(0, g.box_x1 - g.box_x0 + 1), h = std::max(0, g.box_y1 - g.box_y0 + 1);
+  return w * h * 8 <= (int64_t)g.nx * g.ny;
+}
+
 inline int check_omega(double omega) {
   if (!(omega > 0.0 && omega < 2.0)) return set_error(LBM_ERR_OMEGA, "omega must lie in (0, 2)");
   return LBM_OK;

@@ -587,7 +587,8 @@ static int launch_fused(int storage, int flags, const KParams& P, bool overlap, 
   if (!listed) return launch_fused_step(storage, npt, inside, flags, P, overlap, s);
   if (storage == LBM_STORE_F32) {
     // the pass's rows of blocks fit the grid beside the lattice's
-    const bool fits = (int64_t)P.g.ny + P.g.n_bcnodes / kV2Threads + 1 <= 65535;
+    const bool fits = (int64_t)P.g.ny + P.g.n_bcnodes / kV2Threads + 1 <= 65535 &&
+                      (small_box(P.g) || (flags & LBM_FLAG_BC_SPLIT));
     return launch_fused_step(storage, npt, fits ? kBcPass : inside, flags, P, overlap, s);
   }
   if (nodes < ((int64_t)1 << 25) && !(flags & LBM_FLAG_BC_SPLIT))

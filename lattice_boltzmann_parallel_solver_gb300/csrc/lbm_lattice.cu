@@ -522,6 +522,32 @@ static int v2_npt(int storage, int flags, const KParams& P) {
   return npt;
 }
 
+// whether the fixed-point storage has a vectorised kernel of this node count
+// (the cases of launch_fused_step; others take the generic kernel)
+static bool fx_compiled(int npt) { return npt == 1 || npt == 2 || npt == 4; }
+
+// Whether the boundary nodes may be left to the boundary-node pass: the geometry
+// lists them and they are at most an eighth of the lattice; a probe keeps the
+// sources inside the step, so its node is recorded once.
+static bool pass_listed(int npt, int flags, const KParams& P) {
+  return npt > 0 && !(flags & LBM_FLAG_BC_INLINE) && P.g.bcmask != nullptr && P.g.n_bcnodes > 0 &&
+         P.probe_buf == nullptr && (int64_t)P.g.n_bcnodes * 8 <= (int64_t)P.g.nx * P.g.ny;
+}
+
+// whether the pass of a storage other than float32 is a second launch
+static bool pass_apart(int flags, const KParams& P) {
+  return (int64_t)P.g.nx * P.g.ny >= (int64_t)1 << 25 || (flags & LBM_FLAG_BC_SPLIT);
+}
+
+// Whether a run's boundary tables are read as fixed-point numbers: by the
+// vectorised kernels and by the pass.  The generic kernel reads them as float64
+// (before a pass that is a second launch it reads none).
+static bool fx_tables(int storage, int flags, const KParams& P) {
+  const int npt = v2_npt(storage, flags, P);
+  return storage == LBM_STORE_FX64 && npt > 0 &&
+         (fx_compiled(npt) || (pass_listed(npt, flags, P) && pass_apart(flags, P)));
+}
+
 // Lattices that may take several steps per launch: those of the vectorised
 // kernels at their default shape (a flag that picks a one-step kernel or where
 // the boundary sources go keeps the one-step launches).  Under the pressure
@@ -566,9 +592,7 @@ static int launch_fused_step(int storage, int npt, int bc, int flags, const KPar
   }
 }
 
-// One step.  A geometry that lists its boundary nodes (at most an eighth of the
-// lattice) may leave them to the boundary-node pass; a probe keeps the sources
-// inside the step, so its node is recorded once.
+// One step.  The boundary nodes may be left to the boundary-node pass (pass_listed).
 //
 // float32 takes the pass in blocks of the step's own launch, at every size: its
 // body is far from its register cap, and with the sources inside, the warps at a
@@ -580,19 +604,15 @@ static int launch_fused_step(int storage, int npt, int bc, int flags, const KPar
 // as a second launch (8192^2 fx64 1437 against 1444).
 static int launch_fused(int storage, int flags, const KParams& P, bool overlap, cudaStream_t s) {
   const int npt = v2_npt(storage, flags, P);
-  const int64_t nodes = (int64_t)P.g.nx * P.g.ny;
-  const bool listed = npt > 0 && !(flags & LBM_FLAG_BC_INLINE) && P.g.bcmask != nullptr && P.g.n_bcnodes > 0 &&
-                      P.probe_buf == nullptr && (int64_t)P.g.n_bcnodes * 8 <= nodes;
   const int inside = P.g.bcmask != nullptr ? kBcInline : kBcNone;
-  if (!listed) return launch_fused_step(storage, npt, inside, flags, P, overlap, s);
+  if (!pass_listed(npt, flags, P)) return launch_fused_step(storage, npt, inside, flags, P, overlap, s);
   if (storage == LBM_STORE_F32) {
     // the pass's rows of blocks fit the grid beside the lattice's
     const bool fits = (int64_t)P.g.ny + P.g.n_bcnodes / kV2Threads + 1 <= 65535 &&
                       (small_box(P.g) || (flags & LBM_FLAG_BC_SPLIT));
     return launch_fused_step(storage, npt, fits ? kBcPass : inside, flags, P, overlap, s);
   }
-  if (nodes < ((int64_t)1 << 25) && !(flags & LBM_FLAG_BC_SPLIT))
-    return launch_fused_step(storage, npt, inside, flags, P, overlap, s);
+  if (!pass_apart(flags, P)) return launch_fused_step(storage, npt, inside, flags, P, overlap, s);
   KParams Q = P;
   Q.g.bcmask = nullptr;
   if (int e = launch_fused_step(storage, npt, kBcNone, flags, Q, overlap, s)) return e;
@@ -698,7 +718,7 @@ int lbm_lattice_run_opts(const lbm_geometry* g, int32_t storage, void* pop_a, vo
   P.pop_out = pop_b;
   P.aux_in = aux_a;
   P.aux_out = aux_b;
-  if (storage == LBM_STORE_FX64 && v2_npt(storage, flags, P) > 0) set_fx_tables(P.g);
+  if (fx_tables(storage, flags, P)) set_fx_tables(P.g);
   const int tiled_steps = nsteps - (rho_out != nullptr || u_out != nullptr ? 1 : 0);
   TilePlan plan;
   if (tiled_steps >= 3 && tile_applies(storage, flags, P)) plan = tile_plan(storage, P);

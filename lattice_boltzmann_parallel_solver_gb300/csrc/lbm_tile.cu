@@ -114,6 +114,7 @@ TilePlan tile_plan(int storage, const KParams& P) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  best.smem_limit = smem_max;
   const TileCost c = tile_cost(storage, P.g.bcmask != nullptr || P.g.pressure);
   const int nx = P.g.nx, ny = P.g.ny;
   const bool eight = storage == LBM_STORE_F64 || storage == LBM_STORE_FX64;
@@ -160,7 +161,9 @@ TilePlan tile_plan(int storage, const KParams& P) {
 int tile_prepare(int storage, const TilePlan& plan, const KParams& P) {
   const TileKernel k = kernel_of(storage, P, plan.wide);
   if (k == nullptr) return set_error(LBM_ERR_ARG, "unknown storage type");
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
+  // The limit belongs to the kernel, not to this run: the same value whatever the
+  // plan, so that no other thread's run finds it lowered between its launches.
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_limit);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return set_error(LBM_ERR_CUDA, cudaGetErrorString(e));

@@ -13,7 +13,8 @@ namespace lbm {
 struct TilePlan {
   int ksteps = 1, tiles_x = 1, tiles_y = 1, threads = 0;
   bool wide = false;  // regions of up to twice the columns
-  size_t smem = 0;
+  size_t smem = 0;     // shared memory of a launch
+  int smem_limit = 0;  // the most a block of this device may ask for
 };
 
 // the plan for runs of at least three steps of this lattice in this storage

@@ -31,7 +31,8 @@ struct GeoK {
   // reference velocity of the reference-shifted 16-bit storages
   double dev_ref_ux, dev_ref_uy;
   // the frame's descriptors (lbm_geometry; all 0 when it is not given) and the
-  // box of the other boundary nodes (the whole lattice when it is not given)
+  // box of the other boundary nodes (the whole lattice when it is not given, empty
+  // when there are none)
   uint32_t frame_desc[8];
   int box_x0, box_x1, box_y0, box_y1;
 };
@@ -862,12 +863,15 @@ inline bool to_geok(const lbm_geometry* g, GeoK& k) {
     return set_error(LBM_ERR_ARG, "the deviation reference velocity must lie inside (-0.5, 0.5)"), false;
   k.dev_ref_ux = ux;
   k.dev_ref_uy = uy;
-  const bool framed = g->frame != 0 && g->nx >= 3 && g->ny >= 3;
+  // without boundary nodes the box is empty: a batch's chunks then store whole
+  // vectors (with the whole lattice as its box, six 900x400 periodic f32 lattices
+  // took 44.7 us a step instead of 38.7)
+  const bool nodes = k.bcmask != nullptr, framed = nodes && g->frame != 0 && g->nx >= 3 && g->ny >= 3;
   if (framed) std::memcpy(k.frame_desc, g->frame_desc, sizeof(k.frame_desc));
-  k.box_x0 = framed ? g->inner_box[0] : 0;
-  k.box_x1 = framed ? g->inner_box[1] : g->nx - 1;
-  k.box_y0 = framed ? g->inner_box[2] : 0;
-  k.box_y1 = framed ? g->inner_box[3] : g->ny - 1;
+  k.box_x0 = framed ? g->inner_box[0] : (nodes ? 0 : 1);
+  k.box_x1 = framed ? g->inner_box[1] : (nodes ? g->nx - 1 : 0);
+  k.box_y0 = framed ? g->inner_box[2] : (nodes ? 0 : 1);
+  k.box_y1 = framed ? g->inner_box[3] : (nodes ? g->ny - 1 : 0);
   return true;
 }
 

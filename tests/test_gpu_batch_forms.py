@@ -1,0 +1,71 @@
+"""The form a batched step takes follows the storage, the batch's nodes in total
+and where its boundary nodes lie, and every form gives the bits of the step with
+the sources inside its tiles: the boundary-node pass as a launch of its own (two
+launches a step) or in the body's launch (one), with probes on nodes the pass
+records."""
+import numpy as np
+import pytest
+import torch
+
+from lattice_boltzmann_parallel_solver_gb300 import _lib, scenarios
+from lattice_boltzmann_parallel_solver_gb300 import boundary_utils as BU
+from lattice_boltzmann_parallel_solver_gb300.batch import Batch, Member
+from lattice_boltzmann_parallel_solver_gb300.geometry import BOUNCE
+
+pytestmark = pytest.mark.gpu
+
+STEPS = 6
+
+
+def boundary(kind, nx, ny):
+    if kind == "channel":
+        return BU.von_karman_boundary_conditions(nx, ny, 1.0, 0.1, max(6, ny // 5 // 2 * 2), walls=True, plate_offset=1)
+    if kind == "poiseuille":
+        return BU.poiseuille_flow_boundary_conditions(nx, ny, 1.002 / 3, 1 / 3)
+    if kind == "periodic":
+        return None
+
+    def half(nxx, nyy):  # half of a side: no frame
+        m = np.zeros((nxx, nyy), dtype=bool)
+        m[0, : nyy // 2] = True
+        return [(m, i, BOUNCE, 0.001 * i) for i in (2, 5, 6)]
+    return BU.Boundary([BU._Sources(half)])
+
+
+def members(kinds, sizes, storage):
+    out = []
+    for j, (nx, ny) in enumerate(sizes):
+        f, rho, u = scenarios.von_karman_start(nx, ny, u_in=0.05, noise=1e-2, seed=j)
+        kind = kinds[j % len(kinds)]
+        # a wall, a pressure column and an inlet corner: nodes of the pass
+        probe = {"channel": (nx // 3, 0), "poiseuille": (nx - 2, ny // 2), "half": (0, 1)}.get(kind, (1, 1))
+        out.append(Member(nx, ny, 1.2, boundary(kind, nx, ny), steps=STEPS + 1, probe=probe, f0=f, rho0=rho, u0=u, seed=j,
+                          dev_ref=(0.05, 0.0) if storage.endswith("r") else None))
+    return out
+
+
+def check(storage, kinds, sizes, launches, least, blocks=None):
+    """``launches`` a step from ``least`` nodes in total (the sizes hold at least that many)."""
+    runs = []
+    for inline in (True, None):
+        b = Batch(members(kinds, sizes, storage), storage=storage, inline_bc=inline, blocks=blocks).start()
+        assert b.nodes >= least
+        _lib.launches(reset=True)
+        b.run()
+        if inline is None:
+            assert b.bc_chunks >= 0
+            assert _lib.launches() == launches * STEPS + 1  # and the step counter
+        runs.append(b)
+    for j in range(len(sizes)):
+        assert all(torch.equal(x, y) for x, y in zip(runs[0].read(j), runs[1].read(j))), j
+        assert torch.equal(runs[0].probe_trace(j), runs[1].probe_trace(j)), j
+        assert runs[0].probe_trace(j).shape[0] == STEPS
+
+
+MILLION = [(701, 301), (640, 410), (515, 511), (905, 365)]  # 2^20 and 18,315 more
+
+
+@pytest.mark.parametrize("storage", ("f16", "bf16", "f16r", "bf16r"))
+@pytest.mark.parametrize("blocks", (None, 0))
+def test_pass_as_a_second_launch(storage, blocks):
+    check(storage, ("channel", "poiseuille"), MILLION, 2, 1 << 20, blocks)

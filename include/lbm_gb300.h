@@ -299,11 +299,13 @@ size_t lbm_batch_table_bytes(int32_t n);
  * *bc_chunks receives the boundary-node plan that lbm_batch_run takes: -1 when
  * the boundary sources run inside the tiles (some lattice has boundary nodes
  * but no list of them or sets LBM_FLAG_BC_INLINE, or the lattices hold fewer
- * than 2^17 nodes in total and none sets LBM_FLAG_BC_SPLIT), else a positive
- * number that stands for the chunks of `threads` pass nodes: each step is then a
- * boundary-free body over every node and a boundary-node pass over the chunks,
- * in the same launch or, in the 16-bit storages from 2^20 nodes in total, in a
- * second one (bit-identical results, fewer registers in the hot kernel). */
+ * than 2^17 nodes in total and none sets LBM_FLAG_BC_SPLIT; below 2^20 nodes also
+ * when some lattice's boundary nodes off its frame lie in a box of more than an
+ * eighth of it, or it has no frame), else a number >= 0 that stands for the chunks
+ * of `threads` pass nodes: each step is then a boundary-free body over every node
+ * and a boundary-node pass over the chunks, in the same launch or, on larger
+ * batches, in a second one (bit-identical results, fewer registers in the hot
+ * kernel). */
 int lbm_batch_build(const lbm_batch_lattice* lat, int32_t n, int32_t npt, int32_t threads, void* table,
                     size_t table_bytes, int32_t* total_tiles, int32_t* bc_chunks, void* stream);
 /* nsteps batched steps with `blocks` persistent blocks (0 = fill the GPU; more

@@ -83,7 +83,7 @@ int lbm_batch_build(const lbm_batch_lattice* lat, int32_t n, int32_t npt, int32_
       tiles += ((int64_t)e.cpr * e.P.g.ny + run - 1) / run;
     }
   }
-  if (tiles + chunks_bc >= ((int64_t)1 << 31) || chunks_bc >= kPlanMerged)
+  if (tiles + chunks_bc >= ((int64_t)1 << 31) || chunks_bc >= kPlanWide)
     return set_error(LBM_ERR_ARG, "too many tiles");
   // a second copy of the entries for the fixed-point kernels
   for (int j = 0; j < n; ++j) {
@@ -100,7 +100,7 @@ int lbm_batch_build(const lbm_batch_lattice* lat, int32_t n, int32_t npt, int32_
   if (err == cudaSuccess) err = cudaStreamSynchronize((cudaStream_t)stream);
   if (err != cudaSuccess) return set_error(LBM_ERR_CUDA, cudaGetErrorString(err));
   *total_tiles = (int32_t)tiles;
-  *bc_chunks = inline_bc ? -1 : (int32_t)chunks_bc | (nodes < kBatchSplitNodes ? kPlanMerged : 0);
+  *bc_chunks = inline_bc ? -1 : (int32_t)chunks_bc | (wide_box ? kPlanWide : 0) | plan_size(nodes) << kPlanSizeShift;
   return LBM_OK;
 }
 

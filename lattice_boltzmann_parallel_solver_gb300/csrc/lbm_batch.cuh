@@ -1,8 +1,8 @@
 // lbm_batch.cuh -- the batched step kernels and their launcher (many lattices
 // of different sizes advanced together, one or two launches per time step).
-// Two translation units instantiate the launcher: lbm_batch_inline.cu
-// (boundary sources inside the step) and lbm_batch_split.cu (boundary-free
-// step + boundary-node pass).
+// Three translation units instantiate the launcher: lbm_batch_inline.cu
+// (boundary sources inside the step), lbm_batch_split.cu and lbm_batch_split16.cu
+// (boundary-free step + boundary-node pass, the wider and the 16-bit storages).
 #pragma once
 #include <algorithm>
 #include <cstddef>
@@ -164,12 +164,38 @@ __device__ __forceinline__ int owner_of_staged(const int* __restrict__ start, in
 //     caller with 16-bit storages asks for it up to 2^18: 151k nodes 5.7 / 6.0)
 //   from there in the same launch: six 420x180 channels fx64 21.0 / 17.3 / 24.6,
 //     f16 11.6 / 8.9 / 9.8; 1.0M nodes fx64 42.4 / 34.5 / 42.4, f16 19.2 / 13.4 / 14.8
-//   from kBatchSplitNodes the 16-bit storages take the second launch, whose main
-//     body is free of the pass's tests: 1.5M nodes f16 31.3 / 22.5 / 19.8, 4.8M 72 /
-//     55 / 50; the other storages stay (1.5M nodes fx64 60.3 / 50.0 / 57.5)
+//   A launch of its own overwrites what a body free of the pass's tests stored; it
+//     pays on larger batches: the 16-bit storages from 2^20 nodes (1.5M nodes f16
+//     31.3 / 22.5 / 19.8, 4.8M 72 / 55 / 50), fx64 from 2^22 (2.2M channels 78 /
+//     66.2 / 68.1, 4.8M 168 / 140.8 / 138.6, 20M 570 / 563 / 539), f32 from 2^23
+//     (4.8M 94 / 84.6 / 84.9, 12M 182 / 178.6 / 169.8); f64 never (2.2M 297 / 262.7
+//     / 270.0, 40M 4826 / 4831 / 4836).
+//   Where some lattice has a wide box (small_box), whose chunks test and store node
+//     by node beside the pass: inside below 2^20 nodes; from 2^21 f32 and fx64 in a
+//     launch of its own (all such / every second one: f32 1.1M 21.2 / 24.3 / 23.4 and
+//     23.2 / 22.5 / 23.3, 2.2M 39.1 / 47.7 / 43.3 and 40.2 / 43.4 / 43.4, 20M 268 /
+//     340 / 275; fx64 1.6M 55.1 / 55.7 / 56.0, 2.2M 69.5 / 70.0 / 68.3, 20M 548 / 593 /
+//     539); f64, bound by its arithmetic, in the same launch (4.8M 670 / 593 / 599).
+//   Without pass nodes the body is free of the tests as well (periodic, same launch's
+//     body / free one: fx64 20M 560 / 532, f32 12M 172 / 161, f16 0.9M 11.9 / 10.7).
 constexpr int64_t kBatchPassNodes = (int64_t)1 << 17, kBatchSplitNodes = (int64_t)1 << 20;
-// set in the plan of a batch below kBatchSplitNodes
-constexpr int kPlanMerged = 1 << 30;
+
+// A batch's boundary-node plan, from lbm_batch_build to lbm_batch_run: the chunks of
+// pass nodes, whether some lattice has a wide box, and the size class of the nodes in
+// total (0 below 2^20, k below 2^(20 + k), 7 above).
+constexpr int kPlanWide = 1 << 27, kPlanSizeShift = 28;
+inline int plan_size(int64_t nodes) {
+  int k = 0;
+  while (k < 7 && nodes >= kBatchSplitNodes << k) ++k;
+  return k;
+}
+// first size class whose pass is a launch of its own (8: none)
+template <int STORE>
+constexpr int apart_from(bool wide) {
+  if (Store<STORE>::kShifted) return 1;
+  if (STORE == LBM_STORE_F64) return 8;
+  return wide ? 2 : (STORE == LBM_STORE_FX64 ? 3 : 4);
+}
 
 inline int64_t pass_nodes(const GeoK& g) {
   return (g.bcmask != nullptr ? (int64_t)(g.n_bcnodes - g.n_bcnodes_edge) : 0) + (g.pressure ? 2 * (int64_t)g.ny : 0);
@@ -288,9 +314,9 @@ __global__ void __launch_bounds__(THREADS, batch_min_blocks<STORE, NPT, THREADS,
   batch_tile<STORE, NPT, THREADS, HAS_BC, SHIFT, MERGED>(e, tile - __ldg(tile_start + lo), g);
 }
 
-// the pass as a launch of its own
+// the pass as a launch of its own (64 registers; the fixed-point body would spill)
 template <int STORE, int THREADS, bool SHIFT>
-__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
+__global__ void __launch_bounds__(THREADS, STORE == LBM_STORE_FX64 ? 1 : 1024 / THREADS)
     batch_fixup_kernel(const BatchEntry* __restrict__ tab, const int* __restrict__ bc_start, int n_inst,
                        const int* __restrict__ gbase, int k) {
   __shared__ __align__(16) unsigned char ebuf[sizeof(BatchEntry)];
@@ -357,40 +383,44 @@ inline int launch_batch(const void* table, int n, int tiles, int bc_chunks, int*
   if constexpr (HAS_BC) {
     return launch_batch_form<STORE, NPT, THREADS, true, SHIFT, false>(table, n, tiles, 0, gbase, nsteps, blocks, s);
   } else {
-    const int chunks = bc_chunks & ~kPlanMerged;
-    if constexpr (Store<STORE>::kShifted)
-      if (!(bc_chunks & kPlanMerged))
+    const int chunks = bc_chunks & (kPlanWide - 1), size = bc_chunks >> kPlanSizeShift;
+    if constexpr (apart_from<STORE>(true) < 8)
+      if (chunks == 0 || size >= apart_from<STORE>((bc_chunks & kPlanWide) != 0))
         return launch_batch_form<STORE, NPT, THREADS, false, SHIFT, false>(table, n, tiles, chunks, gbase, nsteps, blocks, s);
     return launch_batch_form<STORE, NPT, THREADS, false, SHIFT, true>(table, n, tiles, chunks, gbase, nsteps, blocks, s);
   }
 }
 
-// dispatch over (storage, npt, threads) to launch_batch<..., HAS_BC>
+// dispatch over (storage, npt, threads) to launch_batch<..., HAS_BC>; split16: the
+// 16-bit storages (a translation unit of their own)
 int batch_launch_inline(const void* table, int n, int tiles, int bc_chunks, int storage, int npt, int threads,
                         int* gbase, int nsteps, int blocks, cudaStream_t s);
 int batch_launch_split(const void* table, int n, int tiles, int bc_chunks, int storage, int npt, int threads,
                        int* gbase, int nsteps, int blocks, cudaStream_t s);
+int batch_launch_split16(const void* table, int n, int tiles, int bc_chunks, int storage, int npt, int threads,
+                         int* gbase, int nsteps, int blocks, cudaStream_t s);
 
-#define LBM_BATCH_DISPATCH(HAS_BC)                                                                           \
-  do {                                                                                                       \
-    LBM_BATCH_NPT(LBM_STORE_F64, 2, HAS_BC)                                                                  \
-    LBM_BATCH_NPT(LBM_STORE_F64, 4, HAS_BC)                                                                  \
-    LBM_BATCH_NPT(LBM_STORE_FX64, 1, HAS_BC)                                                                 \
-    LBM_BATCH_NPT(LBM_STORE_FX64, 2, HAS_BC)                                                                 \
-    LBM_BATCH_NPT(LBM_STORE_F32, 2, HAS_BC)                                                                  \
-    LBM_BATCH_NPT(LBM_STORE_F32, 4, HAS_BC)                                                                  \
-    LBM_BATCH_NPT(LBM_STORE_F16S, 2, HAS_BC)                                                                 \
-    LBM_BATCH_NPT(LBM_STORE_F16S, 4, HAS_BC)                                                                 \
-    LBM_BATCH_NPT(LBM_STORE_F16S, 8, HAS_BC)                                                                 \
-    LBM_BATCH_NPT(LBM_STORE_BF16S, 2, HAS_BC)                                                                \
-    LBM_BATCH_NPT(LBM_STORE_BF16S, 4, HAS_BC)                                                                \
-    LBM_BATCH_NPT(LBM_STORE_BF16S, 8, HAS_BC)                                                                \
-    LBM_BATCH_REF(LBM_STORE_F16R, LBM_STORE_F16S, 2, HAS_BC)                                                 \
-    LBM_BATCH_REF(LBM_STORE_F16R, LBM_STORE_F16S, 4, HAS_BC)                                                 \
-    LBM_BATCH_REF(LBM_STORE_BF16R, LBM_STORE_BF16S, 2, HAS_BC)                                               \
-    LBM_BATCH_REF(LBM_STORE_BF16R, LBM_STORE_BF16S, 4, HAS_BC)                                               \
-    return set_error(LBM_ERR_UNSUPPORTED, "no batched kernel for this storage / npt / threads");              \
-  } while (0)
+#define LBM_BATCH_DISPATCH_WIDE(HAS_BC)   \
+  LBM_BATCH_NPT(LBM_STORE_F64, 2, HAS_BC)  \
+  LBM_BATCH_NPT(LBM_STORE_F64, 4, HAS_BC)  \
+  LBM_BATCH_NPT(LBM_STORE_FX64, 1, HAS_BC) \
+  LBM_BATCH_NPT(LBM_STORE_FX64, 2, HAS_BC) \
+  LBM_BATCH_NPT(LBM_STORE_F32, 2, HAS_BC)  \
+  LBM_BATCH_NPT(LBM_STORE_F32, 4, HAS_BC)
+#define LBM_BATCH_DISPATCH_16(HAS_BC)                      \
+  LBM_BATCH_NPT(LBM_STORE_F16S, 2, HAS_BC)                 \
+  LBM_BATCH_NPT(LBM_STORE_F16S, 4, HAS_BC)                 \
+  LBM_BATCH_NPT(LBM_STORE_F16S, 8, HAS_BC)                 \
+  LBM_BATCH_NPT(LBM_STORE_BF16S, 2, HAS_BC)                \
+  LBM_BATCH_NPT(LBM_STORE_BF16S, 4, HAS_BC)                \
+  LBM_BATCH_NPT(LBM_STORE_BF16S, 8, HAS_BC)                \
+  LBM_BATCH_REF(LBM_STORE_F16R, LBM_STORE_F16S, 2, HAS_BC)   \
+  LBM_BATCH_REF(LBM_STORE_F16R, LBM_STORE_F16S, 4, HAS_BC)   \
+  LBM_BATCH_REF(LBM_STORE_BF16R, LBM_STORE_BF16S, 2, HAS_BC) \
+  LBM_BATCH_REF(LBM_STORE_BF16R, LBM_STORE_BF16S, 4, HAS_BC)
+inline int no_batch_kernel() {
+  return set_error(LBM_ERR_UNSUPPORTED, "no batched kernel for this storage / npt / threads");
+}
 #define LBM_BATCH_CASE(ST, NP, TH, HAS_BC)               \
   if (storage == ST && npt == NP && threads == TH)       \
     return launch_batch<ST, NP, TH, HAS_BC>(table, n, tiles, bc_chunks, gbase, nsteps, blocks, s);

@@ -3,6 +3,8 @@ and where its boundary nodes lie, and every form gives the bits of the step with
 the sources inside its tiles: the boundary-node pass as a launch of its own (two
 launches a step) or in the body's launch (one), with probes on nodes the pass
 records."""
+import functools
+
 import numpy as np
 import pytest
 import torch
@@ -32,10 +34,15 @@ def boundary(kind, nx, ny):
     return BU.Boundary([BU._Sources(half)])
 
 
+@functools.lru_cache(maxsize=8)
+def start(nx, ny, seed):
+    return scenarios.von_karman_start(nx, ny, u_in=0.05, noise=1e-2, seed=seed)
+
+
 def members(kinds, sizes, storage):
     out = []
     for j, (nx, ny) in enumerate(sizes):
-        f, rho, u = scenarios.von_karman_start(nx, ny, u_in=0.05, noise=1e-2, seed=j)
+        f, rho, u = start(nx, ny, j % 4)
         kind = kinds[j % len(kinds)]
         # a wall, a pressure column and an inlet corner: nodes of the pass
         probe = {"channel": (nx // 3, 0), "poiseuille": (nx - 2, ny // 2), "half": (0, 1)}.get(kind, (1, 1))
@@ -69,3 +76,25 @@ MILLION = [(701, 301), (640, 410), (515, 511), (905, 365)]  # 2^20 and 18,315 mo
 @pytest.mark.parametrize("blocks", (None, 0))
 def test_pass_as_a_second_launch(storage, blocks):
     check(storage, ("channel", "poiseuille"), MILLION, 2, 1 << 20, blocks)
+
+
+@pytest.mark.parametrize("storage,kinds,sizes,launches,least", [
+    # members without a frame, on both sides of 2^21 nodes
+    ("f32", ("channel", "half"), MILLION, 1, 1 << 20),
+    ("f32", ("half", "channel"), 2 * MILLION, 2, 1 << 21),
+    ("fx64", ("channel", "half"), MILLION, 1, 1 << 20),
+    ("fx64", ("half", "poiseuille"), 2 * MILLION, 2, 1 << 21),
+    ("f64", ("half", "poiseuille"), MILLION, 1, 1 << 20),
+    # framed members, on both sides of 2^22 / 2^23
+    ("fx64", ("channel", "poiseuille"), 2 * MILLION, 1, 1 << 21),
+    ("fx64", ("channel", "poiseuille"), 4 * MILLION, 2, 1 << 22),
+    ("f32", ("channel", "poiseuille"), 4 * MILLION, 1, 1 << 22),
+    ("f32", ("channel", "poiseuille"), 8 * MILLION, 2, 1 << 23),
+    # a few small members in the same launch; members without pass nodes in one
+    ("f16", ("channel", "poiseuille", "periodic"), MILLION[:3], 1, 1 << 18),
+    ("fx64", ("channel", "poiseuille", "periodic"), MILLION[:3], 1, 1 << 18),
+    ("fx64", ("periodic",), 4 * MILLION, 1, 1 << 22),
+    ("f32", ("periodic",), MILLION[:2], 1, 1 << 18),
+    ("f16", ("periodic",), MILLION[:3], 1, 1 << 18)])
+def test_form_by_size(storage, kinds, sizes, launches, least):
+    check(storage, kinds, sizes, launches, least)

@@ -934,8 +934,9 @@ inline void set_fx_tables(GeoK& g) {
 
 // Whether a body that leaves the boundary nodes out finds them cheaply: chunks in
 // the inner box read the mask and store node by node, so the box may hold an
-// eighth of the lattice at most (obstacles all over it, or sides that mix
-// descriptors and so have no frame, keep the sources inside the body)
+// eighth of the lattice at most.  Obstacles all over it, or sides that mix
+// descriptors and so have no frame, keep the sources inside the body or, on large
+// lattices and batches, take the pass as a launch of its own.
 inline bool small_box(const GeoK& g) {
   const int64_t w = std::max(0, g.box_x1 - g.box_x0 + 1), h = std::max(0, g.box_y1 - g.box_y0 + 1);
   return w * h * 8 <= (int64_t)g.nx * g.ny;

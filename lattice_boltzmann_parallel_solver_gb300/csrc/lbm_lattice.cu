@@ -534,9 +534,11 @@ static bool pass_listed(int npt, int flags, const KParams& P) {
          P.probe_buf == nullptr && (int64_t)P.g.n_bcnodes * 8 <= (int64_t)P.g.nx * P.g.ny;
 }
 
-// whether the pass of a storage other than float32 is a second launch
+// whether a pass that is not in the body's launch is a launch of its own (else the
+// sources stay inside)
+constexpr int64_t kApartNodes = (int64_t)1 << 25;
 static bool pass_apart(int flags, const KParams& P) {
-  return (int64_t)P.g.nx * P.g.ny >= (int64_t)1 << 25 || (flags & LBM_FLAG_BC_SPLIT);
+  return (int64_t)P.g.nx * P.g.ny >= kApartNodes || (flags & LBM_FLAG_BC_SPLIT);
 }
 
 // Whether a run's boundary tables are read as fixed-point numbers: by the
@@ -607,10 +609,13 @@ static int launch_fused(int storage, int flags, const KParams& P, bool overlap, 
   const int inside = P.g.bcmask != nullptr ? kBcInline : kBcNone;
   if (!pass_listed(npt, flags, P)) return launch_fused_step(storage, npt, inside, flags, P, overlap, s);
   if (storage == LBM_STORE_F32) {
-    // the pass's rows of blocks fit the grid beside the lattice's
-    const bool fits = (int64_t)P.g.ny + P.g.n_bcnodes / kV2Threads + 1 <= 65535 &&
-                      (small_box(P.g) || (flags & LBM_FLAG_BC_SPLIT));
-    return launch_fused_step(storage, npt, fits ? kBcPass : inside, flags, P, overlap, s);
+    // the pass's rows of blocks fit the grid beside the lattice's; where boundary
+    // nodes are spread over a large lattice, a second launch (5800^2, inside / same
+    // launch / second launch: 396 / 438 / 353)
+    const bool fits = (int64_t)P.g.ny + P.g.n_bcnodes / kV2Threads + 1 <= 65535;
+    const bool large = (int64_t)P.g.nx * P.g.ny >= kApartNodes;
+    if (fits && (small_box(P.g) || ((flags & LBM_FLAG_BC_SPLIT) && !large)))
+      return launch_fused_step(storage, npt, kBcPass, flags, P, overlap, s);
   }
   if (!pass_apart(flags, P)) return launch_fused_step(storage, npt, inside, flags, P, overlap, s);
   KParams Q = P;
@@ -618,6 +623,7 @@ static int launch_fused(int storage, int flags, const KParams& P, bool overlap, 
   if (int e = launch_fused_step(storage, npt, kBcNone, flags, Q, overlap, s)) return e;
   switch (storage) {
     case LBM_STORE_F64: return launch_fixup<LBM_STORE_F64>(P, s);
+    case LBM_STORE_F32: return launch_fixup<LBM_STORE_F32>(P, s);
     case LBM_STORE_F16S: return launch_fixup<LBM_STORE_F16S>(P, s);
     case LBM_STORE_BF16S: return launch_fixup<LBM_STORE_BF16S>(P, s);
     case LBM_STORE_FX64: return launch_fixup<LBM_STORE_FX64>(P, s);

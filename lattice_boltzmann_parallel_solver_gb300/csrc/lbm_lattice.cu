@@ -536,9 +536,10 @@ static bool pass_listed(int npt, int flags, const KParams& P) {
 
 // whether a pass that is not in the body's launch is a launch of its own (else the
 // sources stay inside)
-constexpr int64_t kApartNodes = (int64_t)1 << 25;
-static bool pass_apart(int flags, const KParams& P) {
-  return (int64_t)P.g.nx * P.g.ny >= kApartNodes || (flags & LBM_FLAG_BC_SPLIT);
+constexpr int64_t kApartNodes = (int64_t)1 << 25, kApartNodesShifted = (int64_t)1 << 22;
+static bool pass_apart(int storage, int flags, const KParams& P) {
+  return (int64_t)P.g.nx * P.g.ny >= (ref_shifted(storage) ? kApartNodesShifted : kApartNodes) ||
+         (flags & LBM_FLAG_BC_SPLIT);
 }
 
 // Whether a run's boundary tables are read as fixed-point numbers: by the
@@ -547,7 +548,7 @@ static bool pass_apart(int flags, const KParams& P) {
 static bool fx_tables(int storage, int flags, const KParams& P) {
   const int npt = v2_npt(storage, flags, P);
   return storage == LBM_STORE_FX64 && npt > 0 &&
-         (fx_compiled(npt) || (pass_listed(npt, flags, P) && pass_apart(flags, P)));
+         (fx_compiled(npt) || (pass_listed(npt, flags, P) && pass_apart(storage, flags, P)));
 }
 
 // Lattices that may take several steps per launch: those of the vectorised
@@ -603,7 +604,10 @@ static int launch_fused_step(int storage, int npt, int bc, int flags, const KPar
 // 195 / 178, 8192^2 759 / 698.  In the other storages leaving the nodes out costs
 // the capped body more than the pass saves (4096^2 f16 117 against 107, fx64 377
 // against 367), so they keep the sources inside, and from 2^25 nodes take the pass
-// as a second launch (8192^2 fx64 1437 against 1444).
+// as a second launch (8192^2 fx64 1437 against 1444).  The reference-shifted
+// storages, whose body with sources has the most to hold under its cap, do so from
+// 2^22 (f16r 1500^2 19.4 inside, 20.6 as a second launch, 2049^2 42.5 / 39.3, 5000^2
+// 177.5 / 164.2).
 static int launch_fused(int storage, int flags, const KParams& P, bool overlap, cudaStream_t s) {
   const int npt = v2_npt(storage, flags, P);
   const int inside = P.g.bcmask != nullptr ? kBcInline : kBcNone;
@@ -617,7 +621,7 @@ static int launch_fused(int storage, int flags, const KParams& P, bool overlap, 
     if (fits && (small_box(P.g) || ((flags & LBM_FLAG_BC_SPLIT) && !large)))
       return launch_fused_step(storage, npt, kBcPass, flags, P, overlap, s);
   }
-  if (!pass_apart(flags, P)) return launch_fused_step(storage, npt, inside, flags, P, overlap, s);
+  if (!pass_apart(storage, flags, P)) return launch_fused_step(storage, npt, inside, flags, P, overlap, s);
   KParams Q = P;
   Q.g.bcmask = nullptr;
   if (int e = launch_fused_step(storage, npt, kBcNone, flags, Q, overlap, s)) return e;

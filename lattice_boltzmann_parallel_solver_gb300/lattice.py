@@ -73,9 +73,9 @@ class Lattice:
         deviations stochastically, which keeps increments smaller than half a
         16-bit step from being lost; ``seed`` seeds its random bits.
         In "f32" (in the other storages, or with boundary nodes spread over the
-        lattice, from 2^25 nodes) the vectorised step leaves the boundary nodes
-        to a pass over them; else it applies the boundary sources inside (same
-        results).  ``bc_inline`` True / False
+        lattice, from 2^25 nodes, "f16r" and "bf16r" from 2^22) the vectorised
+        step leaves the boundary nodes to a pass over them; else it applies the
+        boundary sources inside (same results).  ``bc_inline`` True / False
         forces the one or the other.  Small lattices (up to a few hundred
         thousand nodes) take several steps per launch (same results);
         ``bc_inline``, ``npt``, ``generic`` and ``exact`` keep one.  The

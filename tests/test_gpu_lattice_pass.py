@@ -62,3 +62,17 @@ def test_large_lattice_with_spread_nodes(asked):
     assert _lib.launches() == 6
     lats[0].step(3)
     assert all(torch.equal(x, y) for x, y in zip(lats[0].read(), lats[1].read()))
+
+
+@pytest.mark.parametrize("storage,launches", [("f16r", 2), ("bf16r", 2), ("f16", 1)])
+def test_reference_shifted_storages_from_2_22_nodes(storage, launches):
+    nx, ny = 2051, 2047
+    f, rho, u = scenarios.von_karman_start(nx, ny, u_in=0.05, noise=1e-2, seed=3)
+    b = boundary("channel", nx, ny)
+    kw = dict(storage=storage, seed=5, dev_ref=(0.05, 0.0) if storage.endswith("r") else None)
+    lats = [Lattice(nx, ny, 1.3, b, bc_inline=inline, **kw).set_state(f, rho, u).step(1) for inline in (True, None)]
+    _lib.launches(reset=True)
+    lats[1].step(2)
+    assert _lib.launches() == 2 * launches
+    lats[0].step(2)
+    assert all(torch.equal(x, y) for x, y in zip(lats[0].read(), lats[1].read()))

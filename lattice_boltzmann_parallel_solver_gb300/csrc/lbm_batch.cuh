@@ -352,15 +352,19 @@ inline int launch_batch_form(const void* table, int n, int tiles, int bc_chunks,
   const bool plain = (int64_t)blocks * 2 > (int64_t)tiles;
   blocks = std::min(blocks, std::max(1, tiles));
   const int pass = MERGED ? bc_chunks : 0;
+  const bool overlap =
+      plain && tiles > 0
+          ? overlaps<STORE, batch_grid_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT, MERGED>>((int64_t)pass + tiles, THREADS)
+          : overlaps<STORE, batch_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT, MERGED>>((int64_t)pass + blocks, THREADS);
   for (int k = 0; k < nsteps; ++k) {
     if (plain && tiles > 0) {
-      launch_step(batch_grid_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT, MERGED>, dim3((unsigned)(pass + tiles)), THREADS, k > 0,
-                  s, 0, tab, start, n, bc_start, pass, (const int*)gbase, k);
+      launch_step(batch_grid_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT, MERGED>, dim3((unsigned)(pass + tiles)), THREADS,
+                  k > 0 && overlap, s, 0, tab, start, n, bc_start, pass, (const int*)gbase, k);
       count_launch();
       if (int e = check_launch("batch_grid_kernel")) return e;
     } else {
-      launch_step(batch_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT, MERGED>, dim3((unsigned)(pass + blocks)), THREADS, k > 0, s, 0,
-                  tab, start, n, tiles, bc_start, pass, (const int*)gbase, k);
+      launch_step(batch_kernel<STORE, NPT, THREADS, HAS_BC, SHIFT, MERGED>, dim3((unsigned)(pass + blocks)), THREADS,
+                  k > 0 && overlap, s, 0, tab, start, n, tiles, bc_start, pass, (const int*)gbase, k);
       count_launch();
       if (int e = check_launch("batch_kernel")) return e;
     }

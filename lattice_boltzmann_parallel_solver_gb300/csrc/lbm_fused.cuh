@@ -815,6 +815,40 @@ inline void launch_step(void (*kernel)(Params...), dim3 grid, dim3 block, bool o
   cudaLaunchKernelEx(&c, kernel, args...);  // its error is picked up by check_launch
 }
 
+// Whether overlapping the launches of a step kernel pays, `blocks` of them each.
+// Not where it spoils the balance of a kernel bound by the float64 pipe: a plain
+// launch spreads its blocks evenly, ceil(blocks / SMs) of them on an SM at most.  A
+// launch that overlaps the one before it (whose blocks are all resident: at most
+// what the SMs hold) fills the free slots first, and where these do not take all of
+// it the rest follows as slots come free, up to all the slots of one SM.  That costs
+// float64 steps more than the 2 to 4 us of a launch when an even spread leaves a
+// slot free.  us per step, plain / overlapped: 603x162 periodic (3.2 blocks per SM
+// of 5 slots) 22.7 / 25.0, 420x180 Poiseuille (2.4 of 4) 22.6 / 25.1, batches of 1.6 to
+// 2 blocks per SM (of 3) 14.5 / 15.9 to 17.2; outside that range overlapping wins
+// everywhere (2.4 of 5 18.6 / 15.8, 4.0 of 5 26.8 / 25.2).  The other storages gain
+// at every size.
+inline bool overlap_pays(int64_t blocks, int per_sm, int sms) {
+  return blocks > (int64_t)(per_sm - 1) * sms || 2 * blocks <= (int64_t)per_sm * sms;
+}
+// (the resident blocks and the SMs are asked for once per kernel and process)
+template <int STORE, auto KERNEL>
+inline bool overlaps(int64_t blocks, int threads) {
+  if constexpr (STORE != LBM_STORE_F64) return true;
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      cudaGetLastError();
+    return std::max(1, n);
+  }();
+  static const int per_sm = [&] {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, KERNEL, threads, 0) != cudaSuccess) cudaGetLastError();
+    return std::max(1, n);
+  }();
+  return overlap_pays(blocks, per_sm, sms);
+}
+
 // ---- host-side checks shared by the launchers --------------------------------
 inline bool to_geok(const lbm_geometry* g, GeoK& k) {
   if (g == nullptr) return set_error(LBM_ERR_ARG, "geometry is NULL"), false;

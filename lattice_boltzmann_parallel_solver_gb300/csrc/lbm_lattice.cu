@@ -458,23 +458,20 @@ static int launch_read(int storage, bool exact, const KParams& P, double* f, dou
 constexpr int kV2Threads = 128;
 
 // the boundary specialisations of one vectorised kernel; PASS: with kBcPass
-#define LBM_LAUNCH_SPECIALISED(PASS, KERNEL, ...)                                                       \
-  do {                                                                                                  \
-    const bool pr = P.g.pressure != 0;                                                                  \
-    if constexpr (PASS) {                                                                               \
-      if (bc == kBcPass && pr)                                                                          \
-        launch_step(KERNEL<__VA_ARGS__, kBcPass, true>, grid, kV2Threads, overlap, s, 0, P);            \
-      else if (bc == kBcPass)                                                                           \
-        launch_step(KERNEL<__VA_ARGS__, kBcPass, false>, grid, kV2Threads, overlap, s, 0, P);           \
-    }                                                                                                   \
-    if (bc == kBcInline && pr)                                                                          \
-      launch_step(KERNEL<__VA_ARGS__, kBcInline, true>, grid, kV2Threads, overlap, s, 0, P);            \
-    else if (bc == kBcInline)                                                                           \
-      launch_step(KERNEL<__VA_ARGS__, kBcInline, false>, grid, kV2Threads, overlap, s, 0, P);           \
-    else if (bc == kBcNone && pr)                                                                       \
-      launch_step(KERNEL<__VA_ARGS__, kBcNone, true>, grid, kV2Threads, overlap, s, 0, P);              \
-    else if (bc == kBcNone)                                                                             \
-      launch_step(KERNEL<__VA_ARGS__, kBcNone, false>, grid, kV2Threads, overlap, s, 0, P);             \
+#define LBM_LAUNCH_FORM(STORE, BC, PR, KERNEL, ...)                                                                 \
+  launch_step(KERNEL<__VA_ARGS__, BC, PR>, grid, kV2Threads,                                                        \
+              overlap && overlaps<STORE, KERNEL<__VA_ARGS__, BC, PR>>((int64_t)grid.x * grid.y, kV2Threads), s, 0, P)
+#define LBM_LAUNCH_SPECIALISED(PASS, STORE, KERNEL, ...)                                            \
+  do {                                                                                              \
+    const bool pr = P.g.pressure != 0;                                                              \
+    if constexpr (PASS) {                                                                           \
+      if (bc == kBcPass && pr) LBM_LAUNCH_FORM(STORE, kBcPass, true, KERNEL, __VA_ARGS__);          \
+      else if (bc == kBcPass) LBM_LAUNCH_FORM(STORE, kBcPass, false, KERNEL, __VA_ARGS__);          \
+    }                                                                                               \
+    if (bc == kBcInline && pr) LBM_LAUNCH_FORM(STORE, kBcInline, true, KERNEL, __VA_ARGS__);        \
+    else if (bc == kBcInline) LBM_LAUNCH_FORM(STORE, kBcInline, false, KERNEL, __VA_ARGS__);        \
+    else if (bc == kBcNone && pr) LBM_LAUNCH_FORM(STORE, kBcNone, true, KERNEL, __VA_ARGS__);       \
+    else if (bc == kBcNone) LBM_LAUNCH_FORM(STORE, kBcNone, false, KERNEL, __VA_ARGS__);            \
   } while (0)
 
 template <int NPT>
@@ -487,7 +484,7 @@ static int launch_v2(KParams P, int bc, bool overlap, cudaStream_t s) {
   const int bx = v2_blocks<NPT>(P);
   P.pass_rows = bc == kBcPass ? (P.g.n_bcnodes + kV2Threads * bx - 1) / (kV2Threads * bx) : 0;
   const dim3 grid((unsigned)bx, (unsigned)(P.g.ny + P.pass_rows));
-  LBM_LAUNCH_SPECIALISED(STORE == LBM_STORE_F32, fused_v2_kernel, STORE, NPT, kV2Threads, SHIFT);
+  LBM_LAUNCH_SPECIALISED(STORE == LBM_STORE_F32, STORE, fused_v2_kernel, STORE, NPT, kV2Threads, SHIFT);
   count_launch();
   return check_launch("fused_v2_kernel");
 }
@@ -495,7 +492,7 @@ static int launch_v2(KParams P, int bc, bool overlap, cudaStream_t s) {
 template <int NPT>
 static int launch_fx(const KParams& P, int bc, bool overlap, cudaStream_t s) {
   const dim3 grid((unsigned)v2_blocks<NPT>(P), (unsigned)P.g.ny);
-  LBM_LAUNCH_SPECIALISED(false, fused_fx_kernel, NPT, kV2Threads);
+  LBM_LAUNCH_SPECIALISED(false, LBM_STORE_FX64, fused_fx_kernel, NPT, kV2Threads);
   count_launch();
   return check_launch("fused_fx_kernel");
 }

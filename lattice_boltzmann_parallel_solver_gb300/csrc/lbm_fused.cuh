@@ -823,10 +823,11 @@ inline void launch_step(void (*kernel)(Params...), dim3 grid, dim3 block, bool o
 // it the rest follows as slots come free, up to all the slots of one SM.  That costs
 // float64 steps more than the 2 to 4 us of a launch when an even spread leaves a
 // slot free.  us per step, plain / overlapped: 603x162 periodic (3.2 blocks per SM
-// of 5 slots) 22.7 / 25.0, 420x180 Poiseuille (2.4 of 4) 22.6 / 25.1, batches of 1.6 to
-// 2 blocks per SM (of 3) 14.5 / 15.9 to 17.2; outside that range overlapping wins
-// everywhere (2.4 of 5 18.6 / 15.8, 4.0 of 5 26.8 / 25.2).  The other storages gain
-// at every size.
+// of 5 slots) 22.7 / 25.0, 200x450 (3.0 of 5) 18.9 / 25.3, 420x180 Poiseuille (2.4 of 4)
+// 22.6 / 25.1, batches of 1.6 to 2 blocks per SM (of 3) 14.5 / 15.9 to 17.2; outside
+// that range overlapping wins everywhere (2.4 of 5 18.6 / 15.8, 4.03 of 5 26.8 / 25.2).
+// Inside it, a whole number of blocks per SM goes either way (200x456 periodic 18.6 /
+// 15.7, channel 18.6 / 25.2).  The other storages gain at every size.
 inline bool overlap_pays(int64_t blocks, int per_sm, int sms) {
   return blocks > (int64_t)(per_sm - 1) * sms || 2 * blocks <= (int64_t)per_sm * sms;
 }

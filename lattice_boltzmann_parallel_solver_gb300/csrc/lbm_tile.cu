@@ -104,6 +104,21 @@ static TileCost tile_cost(int storage, bool bc) {
   }
 }
 
+// Under the pressure rewrite the 64-bit tile bodies cost more than that (every row of
+// a tile at column 1 or nx-2 runs it): whether the cut that these numbers choose is
+// still faster than a one-step launch, by numbers fitted to the lattices that were
+// tiled without the question (36 in fx64 within 4 percent rms, 31 in f64 within 10).
+// f64's one-step launch, bound by its pipe, counts in whole blocks per SM.  us per
+// step, tiled / one step: fx64 515x230 14.9 / 7.6, 420x180 10.5 / 7.6, 251x132 6.5 / 5.7,
+// 119x168 5.5 / 5.4, 200x60 4.6 / 5.2; f64 251x132 13.4 / 10.8, 267x112 12.4 / 13.8.
+static bool pressure_tile_pays(int storage, const KParams& P, int sms, int ksteps, float trips, float warps) {
+  const int64_t nodes = (int64_t)P.g.nx * P.g.ny;
+  if (storage == LBM_STORE_FX64)
+    return (3.1f + 2.2f * trips + 0.23f * warps) / (float)ksteps < 4.9f + (float)nodes / 39.5e3f;
+  const int64_t blocks = (int64_t)((P.g.nx + 255) / 256) * P.g.ny;  // of 128 threads x 2 nodes
+  return (3.0f + 1.36f * trips + 0.87f * warps) / (float)ksteps < 5.8f + 4.8f * (float)((blocks + sms - 1) / sms);
+}
+
 // The cut with the least time per step: odd numbers of steps, and at most one
 // tile per SM (a second wave never won in a sweep up to 1024^2: by then the
 // one-step launches are bound by their arithmetic, not by their latency, and
@@ -121,6 +136,7 @@ TilePlan tile_plan(int storage, const KParams& P) {
   const int npt = eight || storage == LBM_STORE_F32 ? 1 : 2;
   const int units = (nx + npt - 1) / npt;
   float best_time = c.one_floor + (float)((double)nx * ny / c.one_rate);
+  float best_trips = 0.0f, best_warps = 0.0f;
   for (int k = 3; k <= 7; k += 2) {
     const int margin = 2 * tile_margin_x(k, P.g.pressure != 0);
     for (int tx = 1; tx <= std::min(units, sms); ++tx) {
@@ -139,13 +155,18 @@ TilePlan tile_plan(int storage, const KParams& P) {
       // whole rows, whole warps
       const int row = columns / npt, most = !wide ? 512 : (eight ? 768 : 1024);
       const int threads = (std::min(most, h * row) + 63) / 64 * 64;
-      float time = c.fixed;
+      float time = c.fixed, trips = 0.0f, warps = 0.0f;
       for (int s = 0; s < k; ++s) {
         const int lanes = (h - 2 * s) * row;
-        time += c.trip * (float)((lanes + threads - 1) / threads) + c.warp * (float)((lanes + 31) / 32);
+        const float t = (float)((lanes + threads - 1) / threads), w32 = (float)((lanes + 31) / 32);
+        time += c.trip * t + c.warp * w32;
+        trips += t;
+        warps += w32;
       }
       if (time / (float)k < best_time) {
         best_time = time / (float)k;
+        best_trips = trips;
+        best_warps = warps;
         best.ksteps = k;
         best.tiles_x = tx;
         best.tiles_y = ty;
@@ -155,6 +176,9 @@ TilePlan tile_plan(int storage, const KParams& P) {
       }
     }
   }
+  if (best.ksteps > 1 && P.g.pressure && eight &&
+      !pressure_tile_pays(storage, P, std::max(1, sms), best.ksteps, best_trips, best_warps))
+    best.ksteps = 1;
   return best;
 }
 

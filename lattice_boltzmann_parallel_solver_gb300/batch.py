@@ -85,13 +85,13 @@ class Batch:
         self.inline_bc = inline_bc      # None: chosen by the batch size
         self._auto_shape = (not npt, not threads)
         self.npt, self.threads = int(npt), int(threads)
+        self.members = []
         self._default_shape(0)
         self.blocks = ONE_TILE_PER_BLOCK if blocks is None else blocks
         self.rows = int(rows)           # runs per tile (0: chosen from the batch size)
         self.bc_chunks = -1             # boundary-node plan of the work table (-1: sources in the step)
         self.gbase = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.g = 0                    # host mirror of the global step
-        self.members = []
         for m in members:
             self._alloc(m)
             self.members.append(m)
@@ -161,7 +161,10 @@ class Batch:
         against 16.4 at 2 x 128)."""
         split = not self._inline(nodes)
         if self._auto_shape[0]:
-            self.npt = {"fx64": 1, "f64": 2}.get(self.storage, 4 if split or self.storage == "f32" else 2)
+            # four nodes per thread need six columns
+            narrow = nodes < (1 << 20) and any(m.nx < 6 for m in self.members)
+            wide = split and not narrow or self.storage == "f32"
+            self.npt = {"fx64": 1, "f64": 2}.get(self.storage, 4 if wide else 2)
         if self._auto_shape[1]:
             self.threads = {"fx64": 64 if split else 128}.get(self.storage, 128)
 

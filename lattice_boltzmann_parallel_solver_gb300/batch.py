@@ -155,16 +155,21 @@ class Batch:
         """Default nodes per thread / threads per tile: for the small batches that
         ask for the boundary sources inside (``_inline``) 2 x 128 for the 16-bit
         storages and 1 x 128 for fx64; else 4 x 128 and 1 x 64 (the
-        reference-shifted 16-bit storages as the others), also where the work
-        table puts the sources inside all the same (boundary nodes spread over a
-        lattice: 0.9M nodes fx64 33.5 us a step against 41.0 at 1 x 128, f16 14.4
-        against 16.4 at 2 x 128)."""
+        reference-shifted 16-bit storages as the others).  Where the work table
+        puts the sources inside all the same (``wide_box``), whose tiles are row
+        segments, the 16-bit storages stay at 2 when 4 would leave more lanes
+        past the rows' ends (us a step at 2 and at 4: 0.3M nodes of 64 columns 17.9
+        and 26.0, 0.8M of 420 columns 13.5 and 11.3); fx64's 1 x 64 is the better
+        one there as well (0.9M nodes 33.5, at 1 x 128 41.0)."""
         split = not self._inline(nodes)
         if self._auto_shape[0]:
             # four nodes per thread need six columns
             narrow = nodes < (1 << 20) and any(m.nx < 6 for m in self.members)
-            wide = split and not narrow or self.storage == "f32"
-            self.npt = {"fx64": 1, "f64": 2}.get(self.storage, 4 if wide else 2)
+            four = split and not narrow
+            if four and self.inline_bc is None and nodes < (1 << 20) and any(m.geo.wide_box for m in self.members):
+                lanes = {k: sum(-(-m.nx // (128 * k)) * k * m.ny for m in self.members) for k in (2, 4)}
+                four = lanes[4] <= lanes[2]
+            self.npt = {"fx64": 1, "f64": 2}.get(self.storage, 4 if four or self.storage == "f32" else 2)
         if self._auto_shape[1]:
             self.threads = {"fx64": 64 if split else 128}.get(self.storage, 128)
 

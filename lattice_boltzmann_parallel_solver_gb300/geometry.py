@@ -124,6 +124,17 @@ class CompiledGeometry:
         self.pressure = pressure
         self.struct = g
 
+    @property
+    def wide_box(self) -> bool:
+        """The boundary nodes off the frame lie in a box of more than an eighth of
+        the lattice, or there is no frame: a batch below 2^20 nodes with such a
+        member takes its boundary sources inside the tiles."""
+        g = self.struct
+        if not g.bcmask:
+            return False
+        x0, x1, y0, y1 = g.inner_box if g.frame else (0, self.nx - 1, 0, self.ny - 1)
+        return 8 * max(0, x1 - x0 + 1) * max(0, y1 - y0 + 1) > self.nx * self.ny
+
     @staticmethod
     def _frame(g, nx, ny, nodes, desc):
         """Sets the frame: the one descriptor of each side (without its corners)

@@ -104,3 +104,15 @@ def test_form_by_size(storage, kinds, sizes, launches, least):
 def test_narrow_member(storage, kinds):
     """A lattice too narrow for four nodes per thread in a batch of 2^18 to 2^20 nodes."""
     check(storage, kinds, [(5, 9000), (515, 511)], 1, 1 << 18)
+
+
+@pytest.mark.parametrize("storage", ("f16", "bf16"))
+@pytest.mark.parametrize("kinds,size,count,npt", [
+    (("half",), (64, 700), 7, 2), (("channel", "half"), (200, 250), 6, 2), (("half",), (420, 180), 6, 4),
+    (("channel",), (64, 700), 7, 4), (("periodic",), (64, 700), 7, 4)])
+def test_shape_where_the_sources_stay_inside(storage, kinds, size, count, npt):
+    """Members without a frame keep row-segment tiles: two nodes per thread where
+    four would leave more lanes idle at the rows' ends."""
+    b = Batch(members(kinds, [size] * count, storage), storage=storage).start()
+    assert 1 << 18 <= b.nodes < 1 << 20
+    assert b.npt == npt and (b.bc_chunks == -1) == ("half" in kinds)

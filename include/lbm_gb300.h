@@ -69,12 +69,11 @@ typedef struct lbm_geometry {
   /* device, the n_bcnodes linear indices y*nx + x of the nodes with a bcmask
    * bit.  With it, the vectorised step of the float32 storage, and of the others
    * on lattices of at least 2^25 nodes (the reference-shifted ones 2^22; or with
-   * LBM_FLAG_BC_SPLIT), runs a
-   * boundary-free body over the lattice and recomputes just these nodes with
-   * their sources; NULL, a smaller lattice, more boundary nodes than an eighth of
-   * the lattice, a probe or LBM_FLAG_BC_INLINE applies the sources inside the step,
-   * and so does float32 below 2^25 nodes without the frame below or with an
-   * inner_box of more than an eighth of the lattice. */
+   * LBM_FLAG_BC_SPLIT), runs a boundary-free body over the lattice and recomputes
+   * just these nodes with their sources; NULL, a smaller lattice, more boundary
+   * nodes than an eighth of the lattice, a probe or LBM_FLAG_BC_INLINE applies the
+   * sources inside the step, and so does float32 below 2^25 nodes without the
+   * frame below or with an inner_box of more than an eighth of the lattice. */
   const int32_t* bcnodes;
   int32_t n_bcnodes;
   /* Plain inlet and outlet columns (all zero: none).  edge_inlet_desc is the
@@ -130,7 +129,12 @@ typedef struct lbm_geometry {
 #define LBM_FLAG_BC_SPLIT 2048  /* the boundary-node pass even below the size from which it is taken by default */
 
 /* ---- library ------------------------------------------------------------ */
-int lbm_version(void);
+/* The version of this interface, raised whenever a struct of this header, the size
+ * of a buffer or the meaning of an argument changes: a caller compiled against
+ * another version must not pass its structs.  10100: lbm_geometry has the frame,
+ * the batch work table holds each entry twice, *bc_chunks is a plan. */
+#define LBM_VERSION 10100
+int lbm_version(void); /* LBM_VERSION of the library */
 const char* lbm_last_error(void);
 /* Number of your kernels launched by this thread since the last reset. */
 int64_t lbm_launch_count(int reset);

@@ -33,7 +33,7 @@ void count_launch() { ++g_launches; }
 }  // namespace lbm
 
 extern "C" {
-int lbm_version(void) { return 10000; }
+int lbm_version(void) { return LBM_VERSION; }
 const char* lbm_last_error(void) { return lbm::g_msg; }
 int64_t lbm_launch_count(int reset) {
   int64_t n = lbm::g_launches;

@@ -202,8 +202,8 @@ __global__ void __launch_bounds__(256) lattice_kernel(const __grid_constant__ KP
 }
 
 // The read-out goes from the resident layout (x fastest) to the reference's
-// f[x][y][9] (y fastest).  In the 64-bit storages a tile of kTileX x kTileY nodes
-// passes through shared memory, so that both sides move whole runs (32 elements of
+// f[x][y][9] (y fastest).  On larger lattices of the 64-bit storages (read_tiled) a
+// tile of kTileX x kTileY nodes passes through shared memory, so that both sides move whole runs (32 elements of
 // a plane per row, 576 B of f per column of the tile; a thread that stores its
 // node's 72 B itself takes a sector per population).  The shared rows are 73, 9 and
 // 17 doubles long: odd, so that lanes along x hit different banks.  What is left is
@@ -255,14 +255,23 @@ __global__ void __launch_bounds__(256) init_kernel(const __grid_constant__ KPara
   collide_store<STORE, EXACT>(P, x, y, f, rho, ux, uy);
 }
 
+// Whether a read-out of `nodes` nodes goes through the tile.  Below, the barrier costs
+// more than the whole runs save: us, direct / tiled, with f fx64 64^2 8.4 / 10.5, 420x180
+// 17.9 / 18.1, 640x410 39.2 / 37.7, f64 200x60 5.9 / 7.5, 420x180 15.9 / 15.7; the moments
+// alone f64 420x180 12.9 / 14.7, 1024^2 115.4 / 115.5, 2100x1900 435 / 433.
 template <int STORE>
-constexpr bool read_tiled() { return sizeof(typename Store<STORE>::T) == 8; }
+constexpr bool may_tile_read() { return sizeof(typename Store<STORE>::T) == 8; }
+template <int STORE>
+static bool read_tiled(int64_t nodes, bool with_f) {
+  if (!may_tile_read<STORE>()) return false;
+  return nodes >= (int64_t)1 << (!with_f ? 21 : STORE == LBM_STORE_FX64 ? 17 : 16);
+}
 
 // f_n = BC(stream(S_{n-1})) and its moments in the reference layout (each of the
 // outputs may be null); the moments always follow compute_density /
 // compute_velocity_field exactly.  Blocks of kTileX x kTileY threads in the tiled
 // form, of node_grid otherwise.
-template <int STORE, bool EXACT>
+template <int STORE, bool EXACT, bool TILED>
 __global__ void __launch_bounds__(256) read_kernel(const __grid_constant__ KParams P, double* f_out, double* rho_out,
                                                    double* u_out) {
   using R = typename Store<STORE>::R;
@@ -276,7 +285,7 @@ __global__ void __launch_bounds__(256) read_kernel(const __grid_constant__ KPara
     pull_node<STORE, EXACT>(P, x, y, f);
     node_moments<true>(f, rho, ux, uy);
   }
-  if constexpr (read_tiled<STORE>()) {
+  if constexpr (TILED) {
     __shared__ RefTile t;
     if (in) {
 #pragma unroll
@@ -444,12 +453,18 @@ static int launch_read(int storage, bool exact, const KParams& P, double* f, dou
                        cudaStream_t s) {
   return by_storage(storage, exact, P, [&](const KParams& Q, auto store, auto ex) {
     const int w = (Q.xe > 0 ? Q.xe : Q.g.nx) - Q.xb;
-    dim3 grid, block(kTileX, kTileY);
-    if (read_tiled<store()>())
-      grid = dim3((unsigned)((w + kTileX - 1) / kTileX), (unsigned)((Q.g.ny + kTileY - 1) / kTileY));
-    else
-      node_grid(w, Q.g.ny, grid, block);
-    launch_step(read_kernel<store(), ex()>, grid, block, overlap, s, 0, Q, f, rho, u);
+    dim3 grid, block;
+    if constexpr (may_tile_read<store()>()) {
+      if (read_tiled<store()>((int64_t)w * Q.g.ny, f != nullptr)) {
+        block = dim3(kTileX, kTileY);
+        grid = dim3((unsigned)((w + kTileX - 1) / kTileX), (unsigned)((Q.g.ny + kTileY - 1) / kTileY));
+        launch_step(read_kernel<store(), ex(), true>, grid, block, overlap, s, 0, Q, f, rho, u);
+        count_launch();
+        return check_launch("read_kernel");
+      }
+    }
+    node_grid(w, Q.g.ny, grid, block);
+    launch_step(read_kernel<store(), ex(), false>, grid, block, overlap, s, 0, Q, f, rho, u);
     count_launch();
     return check_launch("read_kernel");
   });

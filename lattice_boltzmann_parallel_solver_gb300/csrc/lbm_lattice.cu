@@ -54,39 +54,39 @@ __device__ __forceinline__ void pull_node(const KParams& P, int x, int y, typena
   const int64_t r0 = (int64_t)y * P.pitch;
   const typename St::A* aux_in = static_cast<const typename St::A*>(P.aux_in);
   auto ld = [&](const T* p, int i) -> R { return node_ld<STORE>(P, p, i); };
-      // pull: direction i arrives from node (x - cx_i, y - cy_i), periodic
-      const int xm = x == 0 ? nx - 1 : x - 1, xp = x == nx - 1 ? 0 : x + 1;
-      const int ym = y == 0 ? ny - 1 : y - 1, yp = y == ny - 1 ? 0 : y + 1;
-      const int64_t rm = (int64_t)ym * P.pitch, rp = (int64_t)yp * P.pitch;
-      const T* pin = static_cast<const T*>(P.pop_in);
-  #pragma unroll
+  // pull: direction i arrives from node (x - cx_i, y - cy_i), periodic
+  const int xm = x == 0 ? nx - 1 : x - 1, xp = x == nx - 1 ? 0 : x + 1;
+  const int ym = y == 0 ? ny - 1 : y - 1, yp = y == ny - 1 ? 0 : y + 1;
+  const int64_t rm = (int64_t)ym * P.pitch, rp = (int64_t)yp * P.pitch;
+  const T* pin = static_cast<const T*>(P.pop_in);
+#pragma unroll
+  for (int i = 0; i < 9; ++i) {
+    const int xs = cx(i) == 1 ? xm : (cx(i) == -1 ? xp : x);
+    const int64_t rs = cy(i) == 1 ? rm : (cy(i) == -1 ? rp : r0);
+    f[i] = ld(pin + i * P.plane + rs + xs, i);
+  }
+  if (P.g.bcmask != nullptr) {
+    const uint32_t word = __ldg(P.g.bcmask + (int64_t)y * P.g.words + (x >> 5));
+    if ((word >> (x & 31)) & 1u) {
+      const uint32_t d = __ldg(P.g.desc + (int64_t)y * nx + x);
+      const int ks = (d >> LBM_DESC_KSET_SHIFT) & 15, cs = (d >> LBM_DESC_CSET_SHIFT) & 15;
+#pragma unroll
       for (int i = 0; i < 9; ++i) {
-        const int xs = cx(i) == 1 ? xm : (cx(i) == -1 ? xp : x);
-        const int64_t rs = cy(i) == 1 ? rm : (cy(i) == -1 ? rp : r0);
-        f[i] = ld(pin + i * P.plane + rs + xs, i);
-      }
-      if (P.g.bcmask != nullptr) {
-        const uint32_t word = __ldg(P.g.bcmask + (int64_t)y * P.g.words + (x >> 5));
-        if ((word >> (x & 31)) & 1u) {
-          const uint32_t d = __ldg(P.g.desc + (int64_t)y * nx + x);
-          const int ks = (d >> LBM_DESC_KSET_SHIFT) & 15, cs = (d >> LBM_DESC_CSET_SHIFT) & 15;
-  #pragma unroll
-          for (int i = 0; i < 9; ++i) {
-            const uint32_t s = (d >> (2 * i)) & 3u;
-            if (s == LBM_SRC_BOUNCE) {
-              const R v = ld(pin + opp(i) * P.plane + r0 + x, opp(i));
-              if (EXACT)
-                f[i] = (R)__dsub_rn((double)v, P.g.kconst[ks][i]);
-              else
-                f[i] = v - (R)P.g.kconst[ks][i];
-            } else if (s == LBM_SRC_CONST) {
-              f[i] = (R)P.g.cconst[cs][i];
-            } else if (s == LBM_SRC_OUTLET && outlet_slot(i) >= 0 && aux_in != nullptr) {
-              f[i] = St::from_aux(aux_in[outlet_slot(i) * ny + y], i);
-            }
-          }
+        const uint32_t s = (d >> (2 * i)) & 3u;
+        if (s == LBM_SRC_BOUNCE) {
+          const R v = ld(pin + opp(i) * P.plane + r0 + x, opp(i));
+          if (EXACT)
+            f[i] = (R)__dsub_rn((double)v, P.g.kconst[ks][i]);
+          else
+            f[i] = v - (R)P.g.kconst[ks][i];
+        } else if (s == LBM_SRC_CONST) {
+          f[i] = (R)P.g.cconst[cs][i];
+        } else if (s == LBM_SRC_OUTLET && outlet_slot(i) >= 0 && aux_in != nullptr) {
+          f[i] = St::from_aux(aux_in[outlet_slot(i) * ny + y], i);
         }
       }
+    }
+  }
 }
 
 // Collides node (x, y) of f_n in place (its moments rho, ux, uy as given) and

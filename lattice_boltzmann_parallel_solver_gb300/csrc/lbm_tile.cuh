@@ -8,14 +8,15 @@
 // populations of the steps between in shared memory, where the computed region
 // shrinks by one node per side and step, and writes the tile back at step K.
 // Neighbouring blocks compute the overlap twice instead of waiting for one
-// another, so no block ever waits for a block.  What bounds it now is the
-// latency of a node's chain on the smallest lattices (0.6 us a step in fx64)
-// and the issue rate above (half of the issue slots used on 420x180).
+// another, so no block ever waits for a block.  What bounds it now is latency on
+// the smallest lattices (64^2 fx64: 1.1 us a step, of which one node's chain 0.6 and
+// the launch's 1.7 us over five steps 0.3) and the issue rate above (half of the issue
+// slots used on 420x180).
 //
-// Measured, us per step, one-step launches -> this: 64^2 fx64 2.2 -> 1.25, f64
-// 6.5 -> 3.0, f32 2.5 -> 0.85, f16 2.4 -> 1.05; 420x180 channel fx64 5.8 -> 3.9,
-// f64 16.3 -> 14.4, f32 5.1 -> 2.5, f16 5.5 -> 2.8; 512^2 cavity f32 6.3 -> 3.7,
-// f16 5.8 -> 4.8; 800x640 cavity f16 8.6 -> 7.2.
+// Measured, us per step, one-step launches -> this: 64^2 fx64 2.2 -> 1.25
+// (1.1 in runs of 2000), f64 6.5 -> 3.0, f32 2.5 -> 0.85, f16 2.4 -> 1.05; 420x180
+// channel fx64 5.8 -> 3.9, f64 16.3 -> 14.4, f32 5.1 -> 2.5, f16 5.5 -> 2.8; 512^2 cavity
+// f32 6.3 -> 3.7, f16 5.8 -> 4.8; 800x640 cavity f16 8.6 -> 7.2.
 //
 // Arithmetic, boundary sources, outlet memory, pressure rewrite, probe and
 // random bits are those of fused_v2_body / fused_fx_body, node for node: the
@@ -308,7 +309,7 @@ __device__ __forceinline__ void tile_body(const KParams& P, const void* pop_in_v
       }
 
       // collision; velocity at the probe's node, pressure rewrite
-      auto probe = [&](int k, double ux, double uy) {
+      auto probe = [&](double ux, double uy) {
         const int q = probe0 + s;
         if (q < P.probe_cap) {
           P.probe_buf[2 * q] = ux;
@@ -338,7 +339,7 @@ __device__ __forceinline__ void tile_body(const KParams& P, const void* pop_in_v
       };
       auto float_extras = [&](int k, R rho, R ux, R uy, const R g[9]) {
         if constexpr (!FX) {
-          if (probed(k)) probe(k, (double)ux, (double)uy);
+          if (probed(k)) probe((double)ux, (double)uy);
           if (pressure_node(k)) {
             R br[9], pv[9];
             bracket9_fast(ux, uy, br);
@@ -358,7 +359,7 @@ __device__ __forceinline__ void tile_body(const KParams& P, const void* pop_in_v
 #pragma unroll
           for (int i = 0; i < 9; ++i) e[i] = fx::from_fx(g[i], wd(i));
           velocity_fast(e, density9(e), ux, uy);
-          probe(0, ux, uy);
+          probe(ux, uy);
         }
         if (pressure_node(0)) {
           int64_t q[9];

@@ -1,7 +1,7 @@
 """Many lattices of different sizes advanced together: one boundary-free
 launch per time step covers every live lattice (a flat list of tiles of
-consecutive node chunks walked by a grid), a second one the boundary nodes,
-optionally replayed from a captured CUDA graph.
+consecutive node chunks walked by a grid), its first blocks or a second launch
+the boundary nodes, optionally replayed from a captured CUDA graph.
 
 This runs what the reference does one driver loop at a time - for example
 the Reynolds / blockage / width sweeps of ``x_strouhal``

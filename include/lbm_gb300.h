@@ -68,12 +68,13 @@ typedef struct lbm_geometry {
   int32_t outlet; /* some node uses LBM_SRC_OUTLET */
   /* device, the n_bcnodes linear indices y*nx + x of the nodes with a bcmask
    * bit.  With it, the vectorised step of the float32 storage, and of the others
-   * on lattices of at least 2^25 nodes (the reference-shifted ones 2^22; or with
-   * LBM_FLAG_BC_SPLIT), runs a boundary-free body over the lattice and recomputes
-   * just these nodes with their sources; NULL, a smaller lattice, more boundary
-   * nodes than an eighth of the lattice, a probe or LBM_FLAG_BC_INLINE applies the
-   * sources inside the step, and so does float32 below 2^25 nodes without the
-   * frame below or with an inner_box of more than an eighth of the lattice. */
+   * on lattices of at least 2^25 nodes (the reference-shifted ones 2^22, without
+   * the frame below 2^24; or with LBM_FLAG_BC_SPLIT), runs a boundary-free body
+   * over the lattice and recomputes just these nodes with their sources; NULL, a
+   * smaller lattice, more boundary nodes than an eighth of the lattice, a probe or
+   * LBM_FLAG_BC_INLINE applies the sources inside the step, and so does float32
+   * below 2^25 nodes without the frame below or with an inner_box of more than an
+   * eighth of the lattice. */
   const int32_t* bcnodes;
   int32_t n_bcnodes;
   /* Plain inlet and outlet columns (all zero: none).  edge_inlet_desc is the

@@ -548,10 +548,11 @@ static bool pass_listed(int npt, int flags, const KParams& P) {
 
 // whether a pass that is not in the body's launch is a launch of its own (else the
 // sources stay inside)
-constexpr int64_t kApartNodes = (int64_t)1 << 25, kApartNodesShifted = (int64_t)1 << 22;
+constexpr int64_t kApartNodes = (int64_t)1 << 25;
 static bool pass_apart(int storage, int flags, const KParams& P) {
-  return (int64_t)P.g.nx * P.g.ny >= (ref_shifted(storage) ? kApartNodesShifted : kApartNodes) ||
-         (flags & LBM_FLAG_BC_SPLIT);
+  const int64_t nodes = (int64_t)P.g.nx * P.g.ny;
+  if (flags & LBM_FLAG_BC_SPLIT) return true;
+  return nodes >= (ref_shifted(storage) ? (int64_t)1 << (small_box(P.g) ? 22 : 24) : kApartNodes);
 }
 
 // Whether a run's boundary tables are read as fixed-point numbers: by the
@@ -618,8 +619,9 @@ static int launch_fused_step(int storage, int npt, int bc, int flags, const KPar
 // against 367), so they keep the sources inside, and from 2^25 nodes take the pass
 // as a second launch (8192^2 fx64 1437 against 1444).  The reference-shifted
 // storages, whose body with sources has the most to hold under its cap, do so from
-// 2^22 (f16r 1500^2 19.4 inside, 20.6 as a second launch, 2049^2 42.5 / 39.3, 5000^2
-// 177.5 / 164.2).
+// 2^22 (f16r cavity 1500^2 19.4 inside, 20.6 as a second launch, 2049^2 42.5 / 39.3,
+// 5000^2 177.5 / 164.2; walls alone 2100^2 40.1 / 37.6), from 2^24 without a frame (half
+// of a side 3000x2600 56.5 / 57.8, 4500^2 139.0 / 133.6).
 static int launch_fused(int storage, int flags, const KParams& P, bool overlap, cudaStream_t s) {
   const int npt = v2_npt(storage, flags, P);
   const int inside = P.g.bcmask != nullptr ? kBcInline : kBcNone;

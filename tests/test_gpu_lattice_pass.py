@@ -76,3 +76,16 @@ def test_reference_shifted_storages_from_2_22_nodes(storage, launches):
     assert _lib.launches() == 2 * launches
     lats[0].step(2)
     assert all(torch.equal(x, y) for x, y in zip(lats[0].read(), lats[1].read()))
+
+
+@pytest.mark.parametrize("storage", ("f16r", "bf16"))
+def test_spread_nodes_stay_inside_at_this_size(storage):
+    nx, ny = 2051, 2047
+    f, rho, u = scenarios.von_karman_start(nx, ny, u_in=0.05, noise=1e-2, seed=3)
+    kw = dict(storage=storage, seed=5, dev_ref=(0.05, 0.0) if storage.endswith("r") else None)
+    lat = Lattice(nx, ny, 1.3, spread(40), **kw).set_state(f, rho, u).step(1)
+    _lib.launches(reset=True)
+    lat.step(2)
+    assert _lib.launches() == 2
+    one = Lattice(nx, ny, 1.3, spread(40), bc_inline=True, **kw).set_state(f, rho, u).step(3)
+    assert all(torch.equal(x, y) for x, y in zip(lat.read(), one.read()))
